@@ -133,7 +133,8 @@ typedef struct lhi_solver_params {   /* SolverParameter<3> (SceneParameter.h:10-
     int32_t smoother;                /* LHI_SMOOTHER_* (0 = reference)         */
     int32_t coarse_cells;            /* MG levels below the finest with at most
                                         this many cells are solved together by
-                                        one CTA in shared memory (0 => 4096)   */
+                                        one thread-block cluster in shared
+                                        memory (0 => every level that fits)    */
     int32_t eager;                   /* 1: the host drives the PCG loop (one
                                         synchronisation per iteration); 0: the
                                         loop runs on the device as a CUDA graph
@@ -344,7 +345,7 @@ LHI_API int lhi_solver_spmv(lhi_liquid* h, double* p_dot_ap, int32_t* tma_kernel
 /* Active tiles of one MG level after the last BuildLHS: tiles of 8 x 8 x 32
    cells (x, y, z) holding a cell with phi <= 0 or covering an active tile of
    the next finer level; the V-cycle and PCG kernels visit only these.
-   Levels solved by the single-CTA coarse kernel report *coarse = 1. */
+   Levels solved by the cluster's coarse kernel report *coarse = 1. */
 LHI_API int lhi_solver_active_tiles(lhi_liquid* h, int32_t level, int32_t* active, int32_t* total,
                                     int32_t* coarse);
 

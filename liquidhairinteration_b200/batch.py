@@ -6,7 +6,7 @@ own CUDA stream, and its pressure solve is one CUDA graph with the PCG loop
 on the device, so one batch step enqueues every scene's whole liquid step
 before the host waits once; the scenes' kernels run concurrently.  An
 autotuner picks, per grid size, the smoother sweeps and the size below which
-the coarse multigrid levels run in one CTA, by the time to solution it
+the coarse multigrid levels run in one cluster, by the time to solution it
 measures on the first scene of that size.  Optionally every solve's
 residuals, cell classes and solution are logged as FP32 training data.
 
@@ -23,7 +23,7 @@ import numpy as np
 from . import abi, scenes
 from ._lib import call
 
-# candidate (pre = post sweeps, coarse-CTA cell limit) the autotuner tries
+# candidate (pre = post sweeps, coarse-cluster cell limit) the autotuner tries
 CANDIDATES = [(1, 512), (2, 512), (2, 4096), (3, 4096)]
 
 

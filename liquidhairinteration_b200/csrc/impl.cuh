@@ -79,9 +79,6 @@ struct SolveScalars {
 // finer level; listed in increasing tile index.
 constexpr int kTileX = 8, kTileY = 8, kTileZ = 32;
 constexpr int kTileThreads = 256;  // 8 warps: warp w takes x = x0 + w, lane = z - z0
-constexpr int kDefaultCoarseCells = 4096;  // levels below the finest this small go to one CTA
-constexpr size_t kCoarseSmemBytes = 224 * 1024;  // shared memory of that CTA
-constexpr int kCoarseThreads = 1024;
 
 struct GridGeom {
     int nx, ny, nz;
@@ -428,11 +425,11 @@ public:
     lhi_solver_params sp_;
     int nlev_;
     LevelDev<T> lv_[kMaxLevels];
-    int coarse_level_ = 0;   // first level solved by the single-CTA coarse kernel (nlev_ if none)
+    int coarse_level_ = 0;   // first level solved by the cluster's coarse kernel (nlev_ if none)
     size_t coarse_smem_ = 0; // its dynamic shared memory
-    uint32_t* coarse_list_ = nullptr;  // per-colour update lists of the coarse levels
-    long long coarse_list_off_[kMaxLevels] = {};
-    int* coarse_counts_ = nullptr;
+    int coarse_ctas_ = 1;    // CTAs of its cluster
+    void* coarse_rows_ = nullptr;  // the coarse levels' rows in the order its threads read them
+    long long coarse_rows_n_ = 0;
     bool spmv_tma_ = false;
     bool fuse_dot_ = false;   // the V-cycle being enqueued is the PCG body's preconditioner
     bool dot_fused_ = false;  // its last level-0 sweep formed r.z, Ap.z and beta

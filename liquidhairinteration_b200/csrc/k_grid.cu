@@ -576,8 +576,7 @@ template <class T, class TX> LiquidImpl<T, TX>::~LiquidImpl() {
         F(lv_[l].tile_flag);
         F(lv_[l].tiles);
     }
-    F(coarse_list_);
-    F(coarse_counts_);
+    F(coarse_rows_);
     if (solve_exec_) cudaGraphExecDestroy(solve_exec_);
     if (tail_exec_) cudaGraphExecDestroy(tail_exec_);
     F(solid_cell_);

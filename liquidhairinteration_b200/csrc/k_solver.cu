@@ -14,9 +14,9 @@
 // an active finer tile so that restricted residuals are carried down).  Cells
 // outside active tiles are air cells whose values no row ever reads.
 //
-// Levels below the finest with at most coarse_cells cells (default 16^3)
-// are solved by one CTA in one launch, staged in shared memory: their
-// pre-smoothing, restriction, coarsest sweeps, prolongation, post-smoothing.
+// The coarse levels whose rows fit the registers of one 16-CTA cluster are
+// solved in one launch, staged in its shared memory: their pre-smoothing,
+// restriction, coarsest sweeps, prolongation, post-smoothing.
 //
 // The PCG loop keeps every scalar on the device.  By default one solve is
 // one CUDA graph: the initial V-cycle, then a conditional while node whose
@@ -921,247 +921,488 @@ __global__ void __launch_bounds__(kTileThreads) k_prolong_t(int fnx, int fny, in
     });
 }
 
-// The coarse levels [first, last] of one V-cycle in a single CTA.
-template <class T> struct CoarseLevels {
+// ------------------------------------------------- coarse levels in a cluster
+// The V-cycle of the coarse levels [first, last] in one launch, on one
+// cluster of up to 16 CTAs.  A level is cut into slabs of x planes, one per
+// CTA; z, r and the residuals live in the CTAs' shared memory, each slab of z
+// with a copy of the neighbouring CTAs' adjacent planes.  Every thread owns
+// at most kSlots cells of each colour of its slab and keeps their rows
+// (diagonal and its reciprocal, six coefficients, r) in registers for all
+// sweeps, so a colour pass loads the neighbours' z from its own shared
+// memory, updates, stores, and pushes the cells of a slab's outer planes
+// into the neighbours' copies through distributed shared memory; a cluster
+// barrier ends the pass.  Levels of one slot a thread run on CTA 0
+// alone, by as many warps as have cells, between CTA barriers: one slot a
+// thread, a pass of 0.3 us against 0.6 us over the cluster (whose barrier
+// with remote stores in flight takes 0.45 us); at 16^3 one CTA's shared
+// memory and issue slots lose (1.0 us a pass against 0.6).
+// What bounds it: the instructions and latency of a pass (shared-memory
+// loads, the update's dependent arithmetic, the barrier), not bytes.  In
+// single precision a thread's slots go in pairs through the packed two-wide
+// multiply-add.  Each update is smooth7's arithmetic in the same order, with
+// the same bits.  Levels 32^3 to 8^3 of a 64^3 dam break, a V-cycle: 41 us
+// with 2+2 sweeps and 20 at the bottom (68 as fused sweeps at 32^3 and one
+// CTA below), 57 us with 5+5 (115).
+namespace cl {
+constexpr int kThreads = 512;
+constexpr int kMaxCtas = 16;
+// cells of one colour per thread: 10 registers of row each, two colours
+// (float: 80 of the 128 registers a 512-thread CTA allows)
+template <class T> constexpr int kSlots = sizeof(T) == 4 ? 4 : 2;
+constexpr size_t kSmemBytes = 216 * 1024;
+// A slot's row in memory: kVecs 16-byte vectors (-d, -c[6], 1 / d) and a
+// word of flags, each kind contiguous over the slots of one colour.
+template <class T> constexpr int kVecs = int(8 * sizeof(T) / 16);
+template <class T> __host__ __device__ constexpr int row_bytes(int items) { return items * (16 * kVecs<T> + 4); }
+// flags: the diagonal is not small (the sweeps update the cell); the slot
+// holds a cell; its plane is the slab's first / last with a neighbour CTA on
+// that side; its diagonal lies outside the range of the division by its
+// reciprocal.  Bits 16 and up: the cell's index in the slab's z.
+constexpr unsigned kUpdate = 1, kCell = 2, kLeft = 4, kRight = 8, kSlow = 16;
+constexpr int kIndexShift = 16;
+}  // namespace cl
+
+template <class T> struct ClusterLevel {
+    int nx, ny, nz;
+    int ctas;    // CTAs of the level: 1 (CTA 0 alone) or the whole cluster
+    int planes;  // x planes per CTA
+    int hz;      // cells of one colour per row, rounded up
+    int items;   // slots of one colour per CTA: planes * ny * hz, rounded up to 4
+    int zoff;    // z in shared memory: planes + 2 planes
+    int roff;    // r in shared memory: planes planes
+    int rowoff;  // the CTA's rows in shared memory, in bytes (-1: they stay in global memory)
+    unsigned char* rows;  // [ctas][2 colours][row_bytes(items)]
+    T* r;
+    T* z;
+};
+
+template <class T> struct ClusterLevels {
     int first, last;
-    LevelK<T> L[kMaxLevels];
-    T* r[kMaxLevels];
-    T* z[kMaxLevels];
-    const uint32_t* list[kMaxLevels];
-    const int* counts;
+    int resoff;  // residuals of the level being restricted, in shared memory
+    int zend;    // end of the levels' z in shared memory
+    ClusterLevel<T> L[kMaxLevels];
 };
 
-// Per-colour lists of the cells a coarse sweep updates (diag not small), one
-// 32-bit entry per cell: index (low 16 bits) | neighbour mask << 16 (bits as
-// the fused sweep's masks).  Built once per BuildLHS by one CTA; counts[2l]
-// ends colour 0 of level l and counts[2l + 1] ends colour 1.
-struct CoarseLists {
-    uint32_t* list[kMaxLevels];
-    int* counts;
-};
-
+// Cell of slot q of a colour: its plane within the slab, y and z.
 template <class T>
-__global__ void __launch_bounds__(1024) k_coarse_lists(CoarseLevels<T> c, CoarseLists cl) {
-    __shared__ int warp_tot[32];
-    __shared__ int base;
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    for (int l = c.first; l <= c.last; ++l) {
-        const LevelK<T>& L = c.L[l];
-        const int n = L.nx * L.ny * L.nz;
-        const int sy = L.nz, sx = L.ny * L.nz;
-        if (threadIdx.x == 0) base = 0;
-        __syncthreads();
-        for (int colour = 0; colour < 2; ++colour) {
-            for (int c0 = 0; c0 < n; c0 += blockDim.x) {
-                const int i = c0 + threadIdx.x;
-                uint32_t ent = 0;
-                int f = 0;
-                if (i < n) {
-                    const int zz = i % L.nz, y = (i / L.nz) % L.ny, x = i / sx;
-                    if (((x + y + zz) & 1) == colour && !is_small(L.diag[i])) {
-                        unsigned m = L.type[i] != 0 ? 64u : 0u;
-                        if (x + 1 < L.nx && L.type[i + sx] == 2) m |= 1u;
-                        if (x > 0 && L.type[i - sx] == 2) m |= 2u;
-                        if (y + 1 < L.ny && L.type[i + sy] == 2) m |= 4u;
-                        if (y > 0 && L.type[i - sy] == 2) m |= 8u;
-                        if (zz + 1 < L.nz && L.type[i + 1] == 2) m |= 16u;
-                        if (zz > 0 && L.type[i - 1] == 2) m |= 32u;
-                        ent = uint32_t(i) | (m << 16);
-                        f = 1;
-                    }
-                }
-                const unsigned bal = __ballot_sync(0xffffffffu, f);
-                if (lane == 0) warp_tot[wp] = __popc(bal);
-                __syncthreads();
-                int off = base;
-                for (int k = 0; k < wp; ++k) off += warp_tot[k];
-                if (f) cl.list[l][off + __popc(bal & ((1u << lane) - 1u))] = ent;
-                __syncthreads();
-                if (threadIdx.x == 0)
-                    for (int k = 0; k < int(blockDim.x >> 5); ++k) base += warp_tot[k];
-                __syncthreads();
+__device__ __forceinline__ bool cluster_slot(const ClusterLevel<T>& L, int cta, int colour, int q, int& p, int& y,
+                                             int& z) {
+    const int row = q / L.hz;
+    p = row / L.ny;
+    y = row - p * L.ny;
+    const int x = cta * L.planes + p;
+    z = 2 * (q - row * L.hz) + ((colour + x + y) & 1);
+    return p < L.planes && x < L.nx && z < L.nz;
+}
+
+// Rows of every cluster level, once per BuildLHS, in slot order: the visits
+// read them coalesced instead of gathering 15 values a cell.
+template <class T> struct ClusterMatrix {
+    LevelK<T> L[kMaxLevels];
+};
+template <class T>
+__global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, ClusterMatrix<T> A) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    int l = c.first;
+    for (; l <= c.last; ++l) {
+        const int n = c.L[l].ctas * 2 * c.L[l].items;
+        if (t < n) break;
+        t -= n;
+    }
+    if (l > c.last) return;
+    const ClusterLevel<T>& C = c.L[l];
+    const LevelK<T>& L = A.L[l];
+    const int half = t / C.items, q = t - half * C.items;  // half: (cta, colour)
+    const int cta = half >> 1, colour = half & 1;
+    const int sy = L.nz, sx = L.ny * L.nz;
+    T w[8] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
+    unsigned m = unsigned(sx) << cl::kIndexShift;  // an empty slot still points into the slab
+    int p, y, z;
+    if (cluster_slot(C, cta, colour, q, p, y, z)) {
+        const int x = cta * C.planes + p;
+        const int i = x * sx + y * sy + z;
+        m = cl::kCell | (unsigned((p + 1) * sx + y * sy + z) << cl::kIndexShift);
+        if (L.type[i] != 0) {  // an air cell's row is empty
+            const T d = L.diag[i];
+            w[0] = -d;
+            if (x + 1 < L.nx && L.type[i + sx] == 2) w[1] = -L.cx[i];
+            if (x > 0 && L.type[i - sx] == 2) w[2] = -L.cx[i - sx];
+            if (y + 1 < L.ny && L.type[i + sy] == 2) w[3] = -L.cy[i];
+            if (y > 0 && L.type[i - sy] == 2) w[4] = -L.cy[i - sy];
+            if (z + 1 < L.nz && L.type[i + 1] == 2) w[5] = -L.cz[i];
+            if (z > 0 && L.type[i - 1] == 2) w[6] = -L.cz[i - 1];
+            if (!is_small(d)) {
+                m |= cl::kUpdate;
+                if (fabs(d) > T(1e-12) && fabs(d) < T(1e12)) w[7] = X<T>::div(T(1), d);
+                else m |= cl::kSlow;
             }
-            if (threadIdx.x == 0) cl.counts[2 * l + colour] = base;
-            __syncthreads();
         }
+        if (C.ctas > 1 && p == 0 && x > 0) m |= cl::kLeft;
+        if (C.ctas > 1 && p == C.planes - 1 && x + 1 < L.nx) m |= cl::kRight;
+    }
+    unsigned char* row = C.rows + size_t(half) * cl::row_bytes<T>(C.items);
+    constexpr int per = 16 / int(sizeof(T));
+#pragma unroll
+    for (int v = 0; v < cl::kVecs<T>; ++v)
+#pragma unroll
+        for (int j = 0; j < per; ++j) reinterpret_cast<T*>(row + (size_t(v) * C.items + q) * 16)[j] = w[v * per + j];
+    reinterpret_cast<uint32_t*>(row + size_t(cl::kVecs<T>) * C.items * 16)[q] = m;
+}
+
+// A thread's slots in groups of W: one value, or two floats in one 64-bit
+// register pair for the packed instructions (each half rounded as the scalar
+// instruction rounds it).
+template <class T, int W> struct Lanes;
+template <class T> struct Lanes<T, 1> {
+    using P = T;
+    static __device__ __forceinline__ P pack(const T* v) { return v[0]; }
+    static __device__ __forceinline__ void unpack(P p, T* v) { v[0] = p; }
+    static __device__ __forceinline__ P mul(P a, P b) { return X<T>::mul(a, b); }
+    static __device__ __forceinline__ P add(P a, P b) { return X<T>::add(a, b); }
+    static __device__ __forceinline__ P fmadd(P a, P b, P c) { return fma(a, b, c); }
+};
+template <> struct Lanes<float, 2> {
+    using P = unsigned long long;
+    static __device__ __forceinline__ P pack(const float* v) {
+        P p;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(v[0]), "f"(v[1]));
+        return p;
+    }
+    static __device__ __forceinline__ void unpack(P p, float* v) {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+    }
+    static __device__ __forceinline__ P mul(P a, P b) {
+        P r;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ P add(P a, P b) {
+        P r;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ P fmadd(P a, P b, P c) {
+        P r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+        return r;
+    }
+};
+
+// The division of the rare operands (see cluster_term).
+template <class T> __device__ __noinline__ T cluster_div(T n, T d) { return X<T>::div(n, d); }
+
+// Rows of a thread's slots: NK of each colour, in groups of W.
+template <class T, int NK> struct ClusterSlots {
+    static constexpr int W = (sizeof(T) == 4 && NK >= 2) ? 2 : 1, G = NK / W;
+    using V = Lanes<T, W>;
+    using P = typename V::P;
+    P nd[2][G], y[2][G], r[2][G], nc[2][G][6];  // -d, 1 / d, r, -c
+    unsigned m[2][NK];
+    __device__ __forceinline__ int a(int c, int k) const { return int(m[c][k] >> cl::kIndexShift); }
+
+    __device__ __forceinline__ void load(const ClusterLevel<T>& L, int cta, const T* __restrict__ sm, bool r_global) {
+        const unsigned char* rows = L.rowoff >= 0 ? reinterpret_cast<const unsigned char*>(sm) + L.rowoff
+                                                  : L.rows + size_t(cta) * 2 * cl::row_bytes<T>(L.items);
+        const int sx = L.ny * L.nz;
+        const T* rg = L.r + (size_t(cta) * L.planes - 1) * sx;
+        const T* rs = sm + L.roff - sx;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const unsigned char* row = rows + c * cl::row_bytes<T>(L.items);
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                T w[W][8], rv[W];
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    const int k = g * W + j, q = int(threadIdx.x) + k * cl::kThreads;
+                    m[c][k] = unsigned(sx) << cl::kIndexShift;  // empty: points into the slab, no flags
+                    rv[j] = T(0);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) w[j][e] = T(0);
+                    if (q >= L.items) continue;
+                    m[c][k] = reinterpret_cast<const uint32_t*>(row + size_t(cl::kVecs<T>) * L.items * 16)[q];
+#pragma unroll
+                    for (int v = 0; v < cl::kVecs<T>; ++v) {
+                        const uint4 u = reinterpret_cast<const uint4*>(row)[v * L.items + q];
+                        memcpy(&w[j][v * (16 / int(sizeof(T)))], &u, 16);
+                    }
+                    if (m[c][k] & cl::kCell) rv[j] = r_global ? rg[a(c, k)] : rs[a(c, k)];
+                }
+                T t[W];
+                auto gather = [&](int e) {
+#pragma unroll
+                    for (int j = 0; j < W; ++j) t[j] = w[j][e];
+                    return V::pack(t);
+                };
+                nd[c][g] = gather(0);
+#pragma unroll
+                for (int e = 0; e < 6; ++e) nc[c][g][e] = gather(1 + e);
+                y[c][g] = gather(7);
+                r[c][g] = V::pack(rv);
+            }
+        }
+    }
+
+    // r - A z of group g of a colour, in ax7's order on negated coefficients (the same roundings); an absent
+    // neighbour adds 0 (its coefficient).  zc: the cells' own z.
+    __device__ __forceinline__ P residual(int c, int g, const T* z, int sx, int sy, P& zc) const {
+        T v[7][W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            const T* p = z + a(c, g * W + j);
+            v[0][j] = p[sx];
+            v[1][j] = p[-sx];
+            v[2][j] = p[sy];
+            v[3][j] = p[-sy];
+            v[4][j] = p[1];
+            v[5][j] = p[-1];
+            v[6][j] = p[0];
+        }
+        zc = V::pack(v[6]);
+        P ax = V::mul(zc, nd[c][g]);
+#pragma unroll
+        for (int e = 0; e < 6; ++e) ax = V::fmadd(V::pack(v[e]), nc[c][g][e], ax);
+        return V::add(r[c][g], ax);
+    }
+
+    // n / d, correctly rounded, from y = 1 / d correctly rounded: two
+    // corrected quotients with exact remainders (P. Markstein, "Computation
+    // of elementary functions on the IBM RISC System/6000 processor", IBM J.
+    // Res. Dev. 34(1), 1990: a quotient within one unit in the last place,
+    // corrected by its exact remainder times the correctly rounded
+    // reciprocal, is the rounded quotient).  Five dependent multiply-adds,
+    // two cells at a time, instead of a division each.  Operands whose
+    // remainders could underflow or overflow take the division.
+    __device__ __forceinline__ P term(int c, int g, P n) const {
+        const P q0 = V::mul(n, y[c][g]);
+        const P q1 = V::fmadd(V::fmadd(nd[c][g], q0, n), y[c][g], q0);
+        P q = V::fmadd(V::fmadd(nd[c][g], q1, n), y[c][g], q1);
+        T nv[W], qv[W], dv[W];
+        V::unpack(n, nv);
+        bool rare = false;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            const T an = fabs(nv[j]);
+            rare |= (!(an > T(1e-18) && an < T(1e18)) && an != T(0)) || (m[c][g * W + j] & cl::kSlow);
+        }
+        if (rare) {
+            V::unpack(q, qv);
+            V::unpack(nd[c][g], dv);
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+                if (m[c][g * W + j] & cl::kUpdate) qv[j] = cluster_div<T>(nv[j], -dv[j]);
+            q = V::pack(qv);
+        }
+        return q;
+    }
+};
+
+// Copies of a slot's z in the neighbouring CTAs' halo planes: the first
+// plane goes after the left CTA's last (which holds `planes` planes), the
+// last one before the right CTA's first.
+struct ClusterSides {
+    uint32_t left, right;  // z index 0's address in the neighbours, moved by the slab
+};
+template <class T>
+__device__ __forceinline__ ClusterSides cluster_sides(const ClusterLevel<T>& L, unsigned rank, const T* z) {
+    ClusterSides o{0, 0};
+    if (L.ctas > 1) {
+        const int slab = L.planes * L.ny * L.nz * int(sizeof(T));
+        if (rank > 0) o.left = map_rank(smem_addr(z), rank - 1) + slab;
+        if (int(rank) + 1 < L.ctas) o.right = map_rank(smem_addr(z), rank + 1) - slab;
+    }
+    return o;
+}
+template <class T> __device__ __forceinline__ void cluster_push(const ClusterSides& o, unsigned m, int a, T v) {
+    if (m & (cl::kLeft | cl::kRight)) {
+        if (m & cl::kLeft) st_cluster(o.left + a * int(sizeof(T)), v);
+        if (m & cl::kRight) st_cluster(o.right + a * int(sizeof(T)), v);
     }
 }
 
-// Sweeps of one level inside the CTA over its colour lists: smooth7's
-// arithmetic in the same order on shared-memory rows.
-template <class T>
-__device__ __forceinline__ void cta_smooth(const LevelK<T>& L, const T* r, T* z, const uint32_t* list, int n0,
-                                           int n01, T w, int variant, int sweeps) {
-    const int sy = L.nz, sx = L.ny * L.nz;
-    constexpr int K = 1;  // cells per colour per thread kept in registers
-    if (n0 <= K * int(blockDim.x) && n01 - n0 <= K * int(blockDim.x)) {
-        // Every thread's cells (at most K per colour) keep diag, r, their six
-        // coefficients and mask in registers for all sweeps; a pass loads
-        // only the neighbours' z.
-        int ci[2][K];
-        unsigned cm[2][K];
-        T cd[2][K], cr[2][K], cf[2][K][6];
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const int e = (c ? n0 : 0) + int(threadIdx.x) + k * int(blockDim.x);
-                ci[c][k] = -1;
-                if (e < (c ? n01 : n0)) {
-                    const uint32_t ent = list[e];
-                    const int i = int(ent & 0xffffu);
-                    ci[c][k] = i;
-                    cm[c][k] = ent >> 16;
-                    cd[c][k] = L.diag[i];
-                    cr[c][k] = r[i];
-                    const unsigned m = cm[c][k];
-                    cf[c][k][0] = (m & 1u) ? L.cx[i] : T(0);
-                    cf[c][k][1] = (m & 2u) ? L.cx[i - sx] : T(0);
-                    cf[c][k][2] = (m & 4u) ? L.cy[i] : T(0);
-                    cf[c][k][3] = (m & 8u) ? L.cy[i - sy] : T(0);
-                    cf[c][k][4] = (m & 16u) ? L.cz[i] : T(0);
-                    cf[c][k][5] = (m & 32u) ? L.cz[i - 1] : T(0);
-                }
+// Ends a step of level l: the cluster's barrier, or that of CTA 0's warps
+// that have cells of the level.  Every level has a CTA barrier of its own:
+// warps without cells of a level wait at the next finer level's barrier
+// meanwhile, and one barrier takes one thread count.
+static_assert(kMaxLevels + 1 <= 16, "a hardware barrier per level beside __syncthreads's");
+__device__ __forceinline__ void cluster_step(bool wide, int l, int threads) {
+    if (wide) cluster_barrier();
+    else asm volatile("bar.sync %0, %1;" ::"r"(l + 1), "r"(threads) : "memory");
+}
+
+constexpr int kVisitDown = 0, kVisitLast = 1, kVisitUp = 2;
+
+// One visit of level l on the way down (smooth, restrict: PressureSolver.cpp:796-819),
+// at the bottom (smooth), or on the way up (prolong: :774-794, smooth).
+// threads: the threads of this CTA that take part (all of them where the level is the cluster's).
+template <class T, int NK>
+__device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int mode, unsigned rank, T* sm, T w,
+                                           int variant, int sweeps, int threads) {
+    using S = ClusterSlots<T, NK>;
+    using V = typename S::V;
+    using P = typename S::P;
+    constexpr int W = S::W, G = S::G;
+    const ClusterLevel<T>& F = c.L[l];
+    const bool wide = F.ctas > 1;
+    const int sy = F.nz, sx = F.ny * F.nz, x0 = int(rank) * F.planes;
+    T* z = sm + F.zoff;
+    const ClusterSides side = cluster_sides(F, rank, z);
+    S s;
+    s.load(F, int(rank), sm, l == c.first);
+    if (mode == kVisitUp) {
+        const ClusterLevel<T>& C = c.L[l + 1];
+        const int csx = C.ny * C.nz;
+        if (C.ctas == 1) cluster_step(wide, l, threads);  // the coarser level is CTA 0's, by fewer warps perhaps
+        // the coarse planes above this slab's planes: C's own z, or copies in place of the residuals
+        const int X0 = x0 >> 1;
+        const T* zc = sm + C.zoff + csx;
+        if (wide) {
+            const int X1 = min(((x0 + F.planes - 1) >> 1) + 1, C.nx);
+            T* copy = sm + c.resoff;
+            for (int i = threadIdx.x; i < (X1 - X0) * csx; i += threads) {
+                const int X = X0 + i / csx, own = C.ctas > 1 ? X / C.planes : 0;
+                copy[i] = ld_cluster<T>(map_rank(smem_addr(zc + (X - own * C.planes) * csx + i % csx), own));
             }
-        for (int s = 0; s < sweeps; ++s)
+            zc = copy;
+            __syncthreads();
+        }
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                T out[K];
+        for (int cc = 0; cc < 2; ++cc)
 #pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const int i = ci[c][k];
-                    if (i < 0) continue;
-                    const unsigned m = cm[c][k];
-                    const T d = cd[c][k];
-                    const T zc = z[i];
-                    T ax = T(0);
-                    if (m & 64u) {
-                        ax = zc * d;
-                        if (m & 1u) ax += z[i + sx] * cf[c][k][0];
-                        if (m & 2u) ax += z[i - sx] * cf[c][k][1];
-                        if (m & 4u) ax += z[i + sy] * cf[c][k][2];
-                        if (m & 8u) ax += z[i - sy] * cf[c][k][3];
-                        if (m & 16u) ax += z[i + 1] * cf[c][k][4];
-                        if (m & 32u) ax += z[i - 1] * cf[c][k][5];
+            for (int k = 0; k < NK; ++k) {
+                if (!(s.m[cc][k] & cl::kCell)) continue;
+                const int a = s.a(cc, k), p = a / sx - 1, rem = a - (p + 1) * sx, y = rem / sy;
+                const int X = (x0 + p) >> 1, Y = y >> 1, Z = (rem - y * sy) >> 1;
+                if (X >= C.nx || Y >= C.ny || Z >= C.nz) continue;
+                const T v = z[a] + zc[(X - X0) * csx + Y * C.nz + Z];
+                z[a] = v;
+                cluster_push(side, s.m[cc][k], a, v);
+            }
+        cluster_step(wide, l, threads);
+    }
+    T wv[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j) wv[j] = w;
+    const P wp = V::pack(wv);
+    const bool busy = int(threadIdx.x & ~31u) < F.items;  // this warp has slots
+    for (int n = 0; n < sweeps; ++n)
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+            if (busy) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    P zc;
+                    const P t = s.term(cc, g, s.residual(cc, g, z, sx, sy, zc));
+                    T out[W];
+                    if (variant == LHI_SMOOTHER_DAMPED_GS) {
+                        V::unpack(V::fmadd(wp, t, zc), out);
+                    } else {
+                        T tv[W], zv[W];
+                        V::unpack(t, tv);
+                        V::unpack(zc, zv);
+#pragma unroll
+                        for (int j = 0; j < W; ++j)
+                            out[j] = T((1.0 - double(w)) * double(zv[j]) + double(X<T>::mul(w, tv[j])));
                     }
-                    const T term = (cr[c][k] - ax) / d;
-                    if (variant == LHI_SMOOTHER_DAMPED_GS) out[k] = zc + w * term;
-                    else out[k] = T((1.0 - double(w)) * double(zc) + double(T(w * term)));
-                }
 #pragma unroll
-                for (int k = 0; k < K; ++k)
-                    if (ci[c][k] >= 0) z[ci[c][k]] = out[k];
-                __syncthreads();
+                    for (int j = 0; j < W; ++j) {
+                        const unsigned m = s.m[cc][g * W + j];
+                        if (m & cl::kUpdate) {
+                            z[s.a(cc, g * W + j)] = out[j];
+                            cluster_push(side, m, s.a(cc, g * W + j), out[j]);
+                        }
+                    }
+                }
             }
+            cluster_step(wide, l, threads);
+        }
+    if (mode != kVisitDown) {
+        T* zg = F.z + (long long)(x0 - 1) * sx;
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+            for (int k = 0; k < NK; ++k)
+                if (s.m[cc][k] & cl::kCell) zg[s.a(cc, k)] = z[s.a(cc, k)];
         return;
     }
-    for (int s = 0; s < sweeps; ++s)
-        for (int colour = 0; colour < 2; ++colour) {
-            const int end = colour ? n01 : n0;
-            for (int e = (colour ? n0 : 0) + int(threadIdx.x); e < end; e += blockDim.x) {
-                const uint32_t ent = list[e];
-                const int i = int(ent & 0xffffu);
-                const unsigned m = ent >> 16;
-                const T d = L.diag[i];
-                const T zc = z[i];
-                T ax = T(0);
-                if (m & 64u) {
-                    ax = zc * d;
-                    if (m & 1u) ax += z[i + sx] * L.cx[i];
-                    if (m & 2u) ax += z[i - sx] * L.cx[i - sx];
-                    if (m & 4u) ax += z[i + sy] * L.cy[i];
-                    if (m & 8u) ax += z[i - sy] * L.cy[i - sy];
-                    if (m & 16u) ax += z[i + 1] * L.cz[i];
-                    if (m & 32u) ax += z[i - 1] * L.cz[i - 1];
-                }
-                const T term = (r[i] - ax) / d;
-                T out;
-                if (variant == LHI_SMOOTHER_DAMPED_GS) out = zc + w * term;
-                else out = T((1.0 - double(w)) * double(zc) + double(T(w * term)));
-                z[i] = out;
-            }
-            __syncthreads();
+    T* res = sm + c.resoff - sx;
+#pragma unroll
+    for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            P zc;
+            T rv[W];
+            V::unpack(s.residual(cc, g, z, sx, sy, zc), rv);
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+                if (s.m[cc][g * W + j] & cl::kCell) res[s.a(cc, g * W + j)] = rv[j];
         }
+    // a coarse plane's children can lie in two slabs where the slabs have an odd number of planes
+    if (wide && !(F.planes & 1)) __syncthreads();
+    else cluster_step(wide, l, threads);
+    // the coarse planes whose first child plane lies in this slab; their r goes to its owner
+    const ClusterLevel<T>& C = c.L[l + 1];
+    const int csx = C.ny * C.nz;
+    const int X0 = (x0 + 1) >> 1, X1 = min((x0 + F.planes + 1) >> 1, C.nx);
+    for (int i = threadIdx.x; i < (X1 - X0) * csx; i += threads) {
+        const int X = X0 + i / csx, rem = i % csx;
+        const int Y = rem / C.nz, Z = rem - Y * C.nz;
+        T rv[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int p = 2 * X + (k >> 2) - x0, fy = 2 * Y + ((k >> 1) & 1), fz = 2 * Z + (k & 1);
+            const bool next = p >= F.planes;
+            const T* src = sm + c.resoff + ((next ? 0 : p) * F.ny + fy) * F.nz + fz;
+            if (next) rv[k] = ld_cluster<T>(map_rank(smem_addr(src), rank + 1));
+            else rv[k] = *src;
+        }
+        T acc = T(0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc = T(double(acc) + 0.125 * double(rv[k]));  // the reference's order
+        const int own = C.ctas > 1 ? X / C.planes : 0;
+        T* dst = sm + C.roff + (X - own * C.planes) * csx + rem;
+        if (own == int(rank)) *dst = acc;
+        else st_cluster(map_rank(smem_addr(dst), own), acc);
+        C.r[X * csx + rem] = acc;
+    }
+    cluster_step(wide, l, threads);  // the next level's r is ready, and no CTA still reads these residuals
 }
 
-// The whole coarse V-cycle in one CTA with every coarse level staged in
-// shared memory: r, z, diag, cx, cy, cz (Scalar) and type per level.
 template <class T>
-__global__ void __launch_bounds__(kCoarseThreads) k_coarse_cycle(CoarseLevels<T> c, T w, int variant, int pre, int post,
-                                                                   int fin, const int* __restrict__ stop) {
-    if (*stop) return;
+__global__ void __launch_bounds__(cl::kThreads, 1)
+    k_coarse_cycle(const __grid_constant__ ClusterLevels<T> c, T w, int variant, int pre, int post, int fin,
+                   const int* __restrict__ stop) {
+    if (*stop) return;  // the same for every CTA: no kernel that sets it runs beside this one
     extern __shared__ __align__(16) unsigned char smem[];
-    LevelK<T> S[kMaxLevels];
-    T* r[kMaxLevels];
-    T* z[kMaxLevels];
-    uint32_t* lst[kMaxLevels];
-    int n0[kMaxLevels], n01[kMaxLevels];
-    size_t off = 0;
+    T* sm = reinterpret_cast<T*>(smem);
+    const unsigned rank = cluster_rank();
+    const bool wide = c.L[c.first].ctas > 1;  // more CTAs than one
+    // the rows that are read from shared memory start on their way (every
+    // thread waits for its own copies before the first barrier)
     for (int l = c.first; l <= c.last; ++l) {
-        const LevelK<T>& G = c.L[l];
-        const int n = G.nx * G.ny * G.nz;
-        T* base = reinterpret_cast<T*>(smem + off);
-        r[l] = base;
-        z[l] = base + n;
-        T* d = base + 2 * n;
-        T* ax = base + 3 * n;
-        T* ay = base + 4 * n;
-        T* az = base + 5 * n;
-        off += size_t(6) * n * sizeof(T);
-        uint8_t* ty = smem + off;
-        off += (size_t(n) + 15) & ~size_t(15);
-        lst[l] = reinterpret_cast<uint32_t*>(smem + off);
-        off += size_t(n) * 4;
-        S[l] = LevelK<T>{G.nx, G.ny, G.nz, d, ax, ay, az, ty};
-        n0[l] = c.counts[2 * l];
-        n01[l] = c.counts[2 * l + 1];
-        for (int e = threadIdx.x; e < n01[l]; e += blockDim.x) lst[l][e] = c.list[l][e];
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            d[i] = G.diag[i];
-            ax[i] = G.cx[i];
-            ay[i] = G.cy[i];
-            az[i] = G.cz[i];
-            ty[i] = G.type[i];
-            r[l][i] = (l == c.first) ? c.r[l][i] : T(0);
-            z[l][i] = (l == c.first) ? c.z[l][i] : T(0);
-        }
+        const ClusterLevel<T>& L = c.L[l];
+        if (L.rowoff < 0 || (L.ctas == 1 && rank != 0)) continue;
+        const int n16 = 2 * cl::row_bytes<T>(L.items) / 16;
+        const unsigned char* src = L.rows + size_t(rank) * 2 * cl::row_bytes<T>(L.items);
+        for (int i = threadIdx.x; i < n16; i += cl::kThreads) copy16_async(smem + L.rowoff + 16 * i, src + 16 * i);
     }
-    __syncthreads();
-    for (int l = c.first; l < c.last; ++l) {
-        cta_smooth(S[l], r[l], z[l], lst[l], n0[l], n01[l], w, variant, pre);
-        const LevelK<T>& C = S[l + 1];
-        const int n = C.nx * C.ny * C.nz;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const int zz = i % C.nz, y = (i / C.nz) % C.ny, x = i / (C.nz * C.ny);
-            restrict_cell(S[l], r[l], z[l], x, y, zz, i, r[l + 1], z[l + 1]);
-        }
-        __syncthreads();
+    for (int i = threadIdx.x; i < c.zend; i += cl::kThreads) sm[i] = T(0);
+    copy_async_wait();
+    if (wide) cluster_barrier();
+    else __syncthreads();
+    const int n = c.last - c.first;
+    for (int step = 0; step <= 2 * n; ++step) {
+        const int l = step <= n ? c.first + step : c.last - (step - n);
+        const int mode = step < n ? kVisitDown : step == n ? kVisitLast : kVisitUp;
+        const int sweeps = mode == kVisitDown ? pre : mode == kVisitLast ? fin : post;
+        const ClusterLevel<T>& L = c.L[l];
+        const int threads = L.ctas > 1 ? cl::kThreads : max(32, min(cl::kThreads, (L.items + 31) & ~31));
+        if ((L.ctas == 1 && rank != 0) || int(threadIdx.x) >= threads) continue;
+        if (L.items <= cl::kThreads) cluster_visit<T, 1>(c, l, mode, rank, sm, w, variant, sweeps, threads);
+        else if (L.items <= 2 * cl::kThreads) cluster_visit<T, 2>(c, l, mode, rank, sm, w, variant, sweeps, threads);
+        else cluster_visit<T, cl::kSlots<T>>(c, l, mode, rank, sm, w, variant, sweeps, threads);
     }
-    cta_smooth(S[c.last], r[c.last], z[c.last], lst[c.last], n0[c.last], n01[c.last], w, variant, fin);
-    for (int l = c.last - 1; l >= c.first; --l) {
-        const LevelK<T>& C = S[l + 1];
-        const LevelK<T>& F = S[l];
-        const int n = C.nx * C.ny * C.nz;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const int zz = i % C.nz, y = (i / C.nz) % C.ny, x = i / (C.nz * C.ny);
-            const T v = z[l + 1][i];
-            const int b = ((x << 1) * F.ny + (y << 1)) * F.nz + (zz << 1);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int f = b + ((k >> 2) & 1) * F.ny * F.nz + ((k >> 1) & 1) * F.nz + (k & 1);
-                z[l][f] = z[l][f] + v;
-            }
-        }
-        __syncthreads();
-        cta_smooth(F, r[l], z[l], lst[l], n0[l], n01[l], w, variant, post);
-    }
-    for (int l = c.first; l <= c.last; ++l) {
-        const int n = S[l].nx * S[l].ny * S[l].nz;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            c.r[l][i] = r[l][i];
-            c.z[l][i] = z[l][i];
-        }
-    }
+    if (wide) cluster_barrier();  // no CTA leaves while another may still reach its shared memory
 }
 
 template <class T>
@@ -1831,23 +2072,6 @@ __global__ void k_loss_grad(LevelK<T> L, const float* __restrict__ e, int batch,
     if (blockIdx.x == 0 && threadIdx.x == 0) red[2] += red[0] / rr / batch;
 }
 
-// The coarse kernel's view of levels [first, nlev): pointers and lists.
-template <class T>
-CoarseLevels<T> coarse_levels_of(const LevelDev<T>* lv, int nlev, int first, uint32_t* list, const long long* off,
-                                 int* counts) {
-    CoarseLevels<T> c{};
-    c.first = first;
-    c.last = nlev - 1;
-    for (int l = first; l < nlev; ++l) {
-        c.L[l] = lk(lv[l]);
-        c.r[l] = lv[l].r;
-        c.z[l] = lv[l].z;
-        c.list[l] = list + off[l];
-    }
-    c.counts = counts;
-    return c;
-}
-
 }  // namespace
 
 // ------------------------------------------------------------- host side
@@ -1955,23 +2179,76 @@ template <class T, class TX> void LiquidImpl<T, TX>::build_lhs(double rho, doubl
     net_type_fresh_ = false;
 }
 
+// The coarse kernel's view of levels [first, nlev): slabs, shared-memory
+// layout, rows.  In shared memory: every level's z, every level's r, the
+// residuals, then the rows of the levels below the first, and the first
+// level's where they still fit (they are read twice a cycle).
+template <class T, class TX> static ClusterLevels<T> coarse_view(const LiquidImpl<T, TX>& s, int first) {
+    ClusterLevels<T> c{};
+    c.first = first;
+    c.last = s.nlev_ - 1;
+    long long off = 4, slab = 0;  // the neighbours of an empty slot may lie just outside its level's z
+    unsigned char* rows = static_cast<unsigned char*>(s.coarse_rows_);
+    for (int l = c.first; l <= c.last; ++l) {
+        const LevelDev<T>& D = s.lv_[l];
+        ClusterLevel<T>& L = c.L[l];
+        L.nx = D.nx;
+        L.ny = D.ny;
+        L.nz = D.nz;
+        L.hz = (D.nz + 1) / 2;
+        // CTA 0 alone where its threads hold the whole level
+        const bool solo = (long long)D.nx * D.ny * L.hz <= cl::kThreads;
+        L.ctas = solo ? 1 : s.coarse_ctas_;
+        L.planes = (D.nx + L.ctas - 1) / L.ctas;
+        L.items = int(std::min(((long long)L.planes * D.ny * L.hz + 3) / 4 * 4, 1LL << 24));
+        L.zoff = int(off);
+        off += (long long)(L.planes + 2) * D.ny * D.nz;
+        L.rows = rows;
+        if (rows) rows += size_t(L.ctas) * 2 * cl::row_bytes<T>(L.items);
+        L.r = D.r;
+        L.z = D.z;
+        slab = std::max(slab, (long long)L.planes * D.ny * D.nz);
+    }
+    off += 4;
+    c.zend = int(off);
+    for (int l = c.first; l <= c.last; ++l) {
+        c.L[l].roff = int(off);
+        off += (long long)c.L[l].planes * c.L[l].ny * c.L[l].nz;
+    }
+    c.resoff = int(off);
+    off = ((off + slab) * (long long)sizeof(T) + 15) / 16 * 16;  // bytes from here on
+    for (int l = c.last; l >= c.first; --l) {
+        const long long bytes = 2LL * cl::row_bytes<T>(c.L[l].items);
+        const bool fits = off + bytes <= (long long)cl::kSmemBytes;
+        c.L[l].rowoff = fits ? int(off) : -1;
+        if (fits) off += bytes;
+    }
+    return c;
+}
+template <class T> static size_t coarse_smem(const ClusterLevels<T>& c) {
+    long long slab = 0, end = 0;
+    for (int l = c.first; l <= c.last; ++l) {
+        const ClusterLevel<T>& L = c.L[l];
+        slab = std::max(slab, (long long)L.planes * L.ny * L.nz);
+        if (L.rowoff >= 0) end = std::max(end, L.rowoff + 2LL * cl::row_bytes<T>(L.items));
+    }
+    return size_t(std::max(end, ((c.resoff + slab) * (long long)sizeof(T) + 15) / 16 * 16));
+}
+
 template <class T, class TX> void LiquidImpl<T, TX>::build_masks() {
-    for (int l = 1; l < nlev_; ++l) {  // level 0's mask comes with its matrix (k_level_matrix)
+    for (int l = 1; l < coarse_level_; ++l) {  // level 0's mask comes with its matrix (k_level_matrix)
         LevelDev<T>& L = lv_[l];
         if (!L.fused) continue;
         k_level_mask<T><<<blocks_for(L.n, 256), 256, 0, cur_>>>(lk(L), L.mask, L.mpitch);
         LHI_LAUNCH_CHECK();
     }
     if (coarse_level_ < nlev_) {
-        CoarseLists cl{};
-        for (int l = coarse_level_; l < nlev_; ++l) cl.list[l] = coarse_list_ + coarse_list_off_[l];
-        cl.counts = coarse_counts_;
-        k_coarse_lists<T><<<1, 1024, 0, cur_>>>(
-            coarse_levels_of(lv_, nlev_, coarse_level_, coarse_list_, coarse_list_off_, coarse_counts_), cl);
+        ClusterMatrix<T> m{};
+        for (int l = coarse_level_; l < nlev_; ++l) m.L[l] = lk(lv_[l]);
+        k_cluster_rows<T><<<blocks_for(coarse_rows_n_, 256), 256, 0, cur_>>>(coarse_view(*this, coarse_level_), m);
         LHI_LAUNCH_CHECK();
     }
 }
-
 
 // Levels that the fused sweep can take: FP32, z extent a multiple of 4 (TMA
 // strides are multiples of 16 bytes), at least 12 cells in x and y and one
@@ -1981,7 +2258,7 @@ template <class T, class TX> void LiquidImpl<T, TX>::setup_fused() {
     if constexpr (std::is_same<T, float>::value) {
         LHI_CUDA(cudaFuncSetAttribute(k_rb_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, rb::kSmem));
         LHI_CUDA(cudaFuncSetAttribute(k_restrict_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, rs::kSmem));
-        for (int l = 0; l < nlev_; ++l) {
+        for (int l = 0; l < coarse_level_; ++l) {  // setup_coarse has run
             LevelDev<T>& L = lv_[l];
             if (L.n == 0 || L.nz % 4 != 0 || L.nx < 12 || L.ny < 12 || L.nz < kTileZ) continue;
             L.mpitch = (L.nz + 15) / 16 * 16;
@@ -2111,40 +2388,57 @@ template <class T, class TX> void LiquidImpl<T, TX>::prolong_to(int level) {
     LHI_LAUNCH_CHECK();
 }
 
-// Bytes of shared memory the coarse kernel needs for levels [first, nlev).
-template <class T> static size_t coarse_bytes(const LevelDev<T>* lv, int first, int nlev) {
-    size_t b = 0;
-    for (int l = first; l < nlev; ++l)
-        b += size_t(6) * lv[l].n * sizeof(T) + ((size_t(lv[l].n) + 15) & ~size_t(15)) + size_t(4) * lv[l].n;
-    return b;
+// CTAs of the coarse kernel's cluster (its non-portable maximum where the
+// device has room for one).
+template <class T> static int coarse_cluster_ctas() {
+    LHI_CUDA(cudaFuncSetAttribute(k_coarse_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cl::kSmemBytes)));
+    LHI_CUDA(cudaFuncSetAttribute(k_coarse_cycle<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int n = cl::kMaxCtas; n > 8; n /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(n));
+        cfg.blockDim = dim3(cl::kThreads);
+        cfg.dynamicSmemBytes = cl::kSmemBytes;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(n);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, k_coarse_cycle<T>, &cfg) == cudaSuccess && fit > 0) return n;
+        cudaGetLastError();
+    }
+    return 8;
 }
 
-// Picks the first level (below the finest) whose cell count is at most
-// coarse_cells and whose coarse V-cycle fits in one CTA's shared memory.
+// Picks the first level (below the finest) from which on every level's slabs
+// fit the cluster: at most coarse_cells cells where the caller set that, and
+// slabs of at most two colours of kSlots cells a thread.
 template <class T, class TX> void LiquidImpl<T, TX>::setup_coarse() {
-    const long long cc = sp_.coarse_cells > 0 ? sp_.coarse_cells : kDefaultCoarseCells;
     coarse_level_ = nlev_;
     coarse_smem_ = 0;
-    for (int l = 1; l < nlev_; ++l) {
-        const size_t b = coarse_bytes(lv_, l, nlev_);
-        if (lv_[l].n <= cc && b <= kCoarseSmemBytes) {
-            coarse_level_ = l;
-            coarse_smem_ = b;
-            break;
-        }
+    if (nlev_ < 2) return;
+    const int ctas = coarse_cluster_ctas<T>();
+    const long long slots = (long long)cl::kSlots<T> * cl::kThreads;
+    for (int first = nlev_ - 1; first >= 1; --first) {  // the finest first level that still fits
+        if (sp_.coarse_cells > 0 && lv_[first].n > sp_.coarse_cells) break;
+        coarse_ctas_ = ctas;
+        const ClusterLevels<T> c = coarse_view(*this, first);
+        if (c.L[first].items > slots || coarse_smem(c) > cl::kSmemBytes) break;
+        coarse_level_ = first;
     }
-    LHI_CUDA(cudaFuncSetAttribute(k_coarse_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(kCoarseSmemBytes)));
-    long long nl = 0;
-    for (int l = coarse_level_; l < nlev_; ++l) {
-        coarse_list_off_[l] = nl;
-        nl += lv_[l].n;
+    if (coarse_level_ == nlev_) return;
+    ClusterLevels<T> c = coarse_view(*this, coarse_level_);
+    coarse_ctas_ = c.L[coarse_level_].ctas;
+    c = coarse_view(*this, coarse_level_);
+    coarse_smem_ = coarse_smem(c);
+    coarse_rows_n_ = 0;
+    size_t bytes = 0;
+    for (int l = c.first; l <= c.last; ++l) {
+        coarse_rows_n_ += 2LL * c.L[l].ctas * c.L[l].items;
+        bytes += size_t(2) * c.L[l].ctas * cl::row_bytes<T>(c.L[l].items);
     }
-    if (coarse_level_ < nlev_) {
-        LHI_CUDA(cudaMalloc(&coarse_list_, sizeof(uint32_t) * size_t(std::max(nl, 1LL))));
-        LHI_CUDA(cudaMalloc(&coarse_counts_, sizeof(int) * 2 * kMaxLevels));
-        LHI_CUDA(cudaMemsetAsync(coarse_counts_, 0, sizeof(int) * 2 * kMaxLevels, stream_));
-    }
+    LHI_CUDA(cudaMalloc(&coarse_rows_, std::max(bytes, size_t(16))));
 }
 
 // CGSolver<3>::ApplyPreconditioner multigrid branch (PressureSolver.cpp:730-771)
@@ -2172,13 +2466,22 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_vcycle_levels() {
             smooth(l, sp_.num_pre_smooth);
             restrict_to(l + 1);
         }
-        const CoarseLevels<T> c =
-            coarse_levels_of(lv_, nlev_, coarse_level_, coarse_list_, coarse_list_off_, coarse_counts_);
         {
             auto ps_ = scope(LHI_KERNEL_SMOOTH_COARSE);
-            k_coarse_cycle<T><<<1, kCoarseThreads, coarse_smem_, cur_>>>(c, T(sp_.smoothing_factor), sp_.smoother,
-                                                                sp_.num_pre_smooth, sp_.num_post_smooth,
-                                                                sp_.num_final_smooth, &sc_->stop);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(unsigned(coarse_ctas_));
+            cfg.blockDim = dim3(cl::kThreads);
+            cfg.dynamicSmemBytes = coarse_smem_;
+            cfg.stream = cur_;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = unsigned(coarse_ctas_);
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            LHI_CUDA(cudaLaunchKernelEx(&cfg, k_coarse_cycle<T>, coarse_view(*this, coarse_level_), T(sp_.smoothing_factor),
+                                        int(sp_.smoother), int(sp_.num_pre_smooth), int(sp_.num_post_smooth),
+                                        int(sp_.num_final_smooth), static_cast<const int*>(&sc_->stop)));
             LHI_LAUNCH_CHECK();
         }
         for (int l = Lc - 1; l >= 0; --l) {

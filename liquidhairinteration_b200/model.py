@@ -312,7 +312,7 @@ class CGSolver:
         return n.value
 
     def ActiveTiles(self, level=0):
-        """(active tiles, total tiles, solved by the coarse CTA) of a level."""
+        """(active tiles, total tiles, solved by the coarse cluster) of a level."""
         a, t, c = C.c_int32(), C.c_int32(), C.c_int32()
         call("lhi_solver_active_tiles", self._m._h, int(level), C.byref(a), C.byref(t), C.byref(c))
         return a.value, t.value, bool(c.value)
