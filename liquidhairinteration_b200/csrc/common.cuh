@@ -161,6 +161,60 @@ template <class T> __device__ __forceinline__ T dot3(T a0, T a1, T a2, T b0, T b
     return X<T>::add(X<T>::mul(a0, b0), X<T>::add(X<T>::mul(a1, b1), X<T>::mul(a2, b2)));
 }
 
+// ------------------------------------------------------- packed arithmetic
+// W values of T in one operand: two floats go in a 64-bit register pair
+// through the packed instructions (half the issue slots; each half rounded as
+// the scalar instruction rounds it).
+template <class T, int W> struct Lanes;
+template <class T> struct Lanes<T, 1> {
+    using P = T;
+    static __device__ __forceinline__ P pack(const T* v) { return v[0]; }
+    static __device__ __forceinline__ void unpack(P p, T* v) { v[0] = p; }
+    static __device__ __forceinline__ P mul(P a, P b) { return X<T>::mul(a, b); }
+    static __device__ __forceinline__ P add(P a, P b) { return X<T>::add(a, b); }
+    static __device__ __forceinline__ P fmadd(P a, P b, P c) { return fma(a, b, c); }
+};
+template <> struct Lanes<float, 2> {
+    using P = unsigned long long;
+    static __device__ __forceinline__ P pack(const float* v) {
+        P p;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(v[0]), "f"(v[1]));
+        return p;
+    }
+    static __device__ __forceinline__ void unpack(P p, float* v) {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+    }
+    static __device__ __forceinline__ P mul(P a, P b) {
+        P r;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ P add(P a, P b) {
+        P r;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ P fmadd(P a, P b, P c) {
+        P r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+        return r;
+    }
+};
+
+template <> struct Lanes<double, 2> {
+    using P = double2;
+    static __device__ __forceinline__ P pack(const double* v) { return make_double2(v[0], v[1]); }
+    static __device__ __forceinline__ void unpack(P p, double* v) {
+        v[0] = p.x;
+        v[1] = p.y;
+    }
+    static __device__ __forceinline__ P mul(P a, P b) { return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)); }
+    static __device__ __forceinline__ P add(P a, P b) { return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)); }
+    static __device__ __forceinline__ P fmadd(P a, P b, P c) {
+        return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+    }
+};
+
 // ------------------------------------------------------------ reductions
 template <class T> __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

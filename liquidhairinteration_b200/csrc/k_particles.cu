@@ -341,18 +341,6 @@ template <class T> __device__ __forceinline__ void axis_weights(T t, T w[3], T g
     gw[2] = -r;
 }
 
-// LiquidModel<3>::Particle2Grid accumulation (LiquidModel.cpp:614-701).
-// One CTA per 8^3-cell tile.  Thread t owns cells t and t + 256 of the tile;
-// for each face component it walks its cell's sorted particles and sums
-// their weights and APIC values for the cell's fixed window of nodes (4
-// along the component's axis, offsets -1..2; 3 across, offsets -1..1) in
-// registers, then adds each window node once into the tile's shared-memory
-// accumulators.  The lanes of a warp own distinct cells, so at any step they
-// add to distinct nodes.  Finally each touched node goes to global memory
-// with one add.  The per-axis weights and C.(x_p - x_node) terms are the
-// reference's, rounded the same way; the per-node products are regrouped
-// and fused (multiply-add), and particles are summed in another order, so
-// P2G matches the reference to rounding, not bit for bit.
 // A particle whose own truncated index (cast<Integer>, LiquidModel.cpp:629)
 // is not the cell it was sorted into (only outside the grid, where the sort
 // key is clamped) adds its window straight to global memory.
@@ -411,46 +399,47 @@ __host__ __device__ constexpr int p2g_region(int a) {
     return (kTile + 2 + (a == 0)) * (kTile + 2 + (a == 1)) * (kTile + 2 + (a == 2));
 }
 
-// Staged particle records of the P2G warp loop (values of T), two per
-// particle:
-//   A (kP2GRecA values, 16-byte aligned: the lanes read wf and tf as vectors)
-//     [0, 12)   wf[a][4]: face weights of component a along its own axis,
-//               window slots -1..2 (node = cell + slot)
-//     [12, 24)  tf[a][4] = C_aa * (x_a - face node a)
-//     [24, 28)  unused (padding to 16 bytes)
-//   B (kP2GRecB values, odd stride: the staging lanes' stores fall in
-//     distinct banks)
-//     [0, 27)   W[l], column l = 9a + 3s + t of the warp loop: the product of
-//               the two cell-centre weights across component a (slot s on its
-//               first other axis, t on the second; node centre = cell + slot + 0.5)
-//     [27, 54)  B[l] = v_a + C_ab (x_b - centre b) + C_ac (x_c - centre c)
+// Staged particle record of the P2G warp loop (kP2GRec values of T, 16-byte
+// aligned vectors):
+//   [8a, 8a + 4)       wf: face weights of component a along its own axis,
+//                      window slots -1..2 (node = cell + slot)
+//   [8a + 4, 8a + 8)   wf * C_aa (x_a - face node)
+//   [24 + 12a, + 6)    (weight, C_ac (x_c - centre)) of component a's second
+//                      other axis c, slots -1..1 (centre = cell + slot + 0.5)
+//   [30 + 12a, + 6)    (weight, v_a + C_ab (x_b - centre)) of its first other
+//                      axis b
 // The weights are the quadratic B-spline's in closed form around the
 // particle's middle node (axis_weights); a node outside the reference's
 // window (+-d) gets 0, as does a node at |e| >= 1.5 by the formula itself.
-constexpr int kP2GRecA = 28;
-constexpr int kP2GRecB = 55;
+constexpr int kP2GRec = 60;
 constexpr int kP2GWarps = 8;
-constexpr int kP2GChunk = 16;  // particles staged at a time per warp
-constexpr int kP2GStage = kP2GChunk * (kP2GRecA + kP2GRecB);  // values per warp
+constexpr int kP2GChunk = 24;  // particles staged at a time per warp: three CTAs fit an SM
+constexpr int kP2GStage = kP2GChunk * kP2GRec;  // values per warp
 
 __device__ __forceinline__ void p2g_other_axes(int a, int& b, int& c) {
     b = (a == 0) ? 1 : 0;
     c = (a == 2) ? 1 : 2;
 }
 
-__device__ __forceinline__ void load4(const float* p, float v[4]) {
-    const float4 t = *reinterpret_cast<const float4*>(p);
+__device__ __forceinline__ void load2(const float* p, float v[2]) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
     v[0] = t.x;
     v[1] = t.y;
-    v[2] = t.z;
-    v[3] = t.w;
 }
-__device__ __forceinline__ void load4(const double* p, double v[4]) {
-    const double2 t0 = reinterpret_cast<const double2*>(p)[0], t1 = reinterpret_cast<const double2*>(p)[1];
-    v[0] = t0.x;
-    v[1] = t0.y;
-    v[2] = t1.x;
-    v[3] = t1.y;
+__device__ __forceinline__ void load2(const double* p, double v[2]) {
+    const double2 t = *reinterpret_cast<const double2*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+}
+// four values as two packed pairs (16-byte aligned)
+__device__ __forceinline__ void load_pairs(const float* p, unsigned long long v[2]) {
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+}
+__device__ __forceinline__ void load_pairs(const double* p, double2 v[2]) {
+    v[0] = reinterpret_cast<const double2*>(p)[0];
+    v[1] = reinterpret_cast<const double2*>(p)[1];
 }
 __device__ __forceinline__ void store4(float* p, const float v[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
@@ -460,118 +449,163 @@ __device__ __forceinline__ void store4(double* p, const double v[4]) {
     reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
-// Computes the records of one particle (one lane per particle) and returns
-// the z offset of its cell in the row, or -1 when its own truncated index
+// One particle's state as it is staged.
+template <class T> struct P2GParticle {
+    T q[3], v[3], C[9];  // C column-major: C[3a + i] = C(i, a)
+};
+
+template <class T>
+__device__ __forceinline__ void p2g_fetch(const PView<T>& pv, long long p, P2GParticle<T>& s) {
+    const long long ps = pv.order ? (long long)pv.order[p] : p;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s.q[i] = pv.pos[i * pv.cap + p];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s.v[i] = pv.rest[(3 + i) * pv.cap + ps];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) s.C[i] = pv.rest[(6 + i) * pv.cap + ps];
+}
+
+// Writes the record of one particle (one lane per particle) and returns the
+// z offset of its cell in the row, or -1 when its own truncated index
 // (cast<Integer>, LiquidModel.cpp:629) is not the cell it was sorted into,
 // or its grid coordinate is negative (both only outside the grid, where the
 // sort key is clamped): such a particle is listed for k_p2g_overflow.
 template <class T>
-__device__ int p2g_stage(const GridP<T>& g, int d0, int d1, int d2, const PView<T>& pv, long long p, int rx, int ry,
-                         int z0, int zend, T* ra, T* rb, int* __restrict__ ov_count, int32_t* __restrict__ ov_list) {
-    const long long cap = pv.cap;
-    const T q[3] = {pv.pos[p], pv.pos[cap + p], pv.pos[2 * cap + p]};
-    T g3[3];
+__device__ __forceinline__ int p2g_stage(const GridP<T>& g, const int dd[3], const P2GParticle<T>& s, long long p,
+                                         int rx, int ry, int z0, int zend, T* rec, int* __restrict__ ov_count,
+                                         int32_t* __restrict__ ov_list) {
+    const bool clip = dd[0] < 2 || dd[1] < 2 || dd[2] < 2;  // the window ends inside the spline's support
+    T f[3];
     int ci[3];
+    bool in = true;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         // cwiseQuotient as a multiply (P2G equals the reference up to rounding; a particle whose cell then
         // differs from its sort key's takes the overflow path, which divides)
-        g3[i] = (q[i] - g.mn[i]) * g.idx[i];
-        ci[i] = int(g3[i]);  // cast<Integer>
+        const T g3 = (s.q[i] - g.mn[i]) * g.idx[i];
+        ci[i] = int(g3);  // cast<Integer>
+        in = in && g3 >= T(0);
+        f[i] = g3 - T(ci[i]);  // exact, in [0, 1)
     }
-    if (ci[0] != rx || ci[1] != ry || ci[2] < z0 || ci[2] >= zend ||
-        !(g3[0] >= T(0) && g3[1] >= T(0) && g3[2] >= T(0))) {
+    if (!in || ci[0] != rx || ci[1] != ry || ci[2] < z0 || ci[2] >= zend) {
         ov_list[atomicAdd(ov_count, 1)] = int32_t(p);
         return -1;
     }
-    const long long ps = pv.order ? (long long)pv.order[p] : p;
-    T C[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) C[k] = pv.rest[(6 + k) * cap + ps];  // column-major: C[3a + i] = C(i, a)
-    const int dd[3] = {d0, d1, d2};
-    T wc[3][3], tc[3][2][3];  // centre weights per axis; C_ab (x_b - centre) per component and other axis
+    T pair[3][12];  // per component: 6 values of axis c, then 6 of axis b
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const T cb = T(ci[i]);  // integer grid coordinates are exact in T
-        const T f = g3[i] - cb;  // exact, in [0, 1)
-        const bool up = f >= T(0.5f);
-        T w3[3], gu[3];
-        axis_weights(g3[i] - (up ? cb + T(1) : cb), w3, gu);  // face nodes: middle node = nearest integer
-        T wf[4], tf[4];
+        T w3[3], gu[3], wf[4], uf[4];
+        const bool up = f[i] >= T(0.5f);
+        axis_weights(f[i] - (up ? T(1) : T(0)), w3, gu);  // face nodes: middle node = nearest integer
+        const T ci = s.C[4 * i] * g.dx[i];
 #pragma unroll
-        for (int s2 = 0; s2 < 4; ++s2) {  // slot s2 = offset + 1 from the cell
-            const int o = s2 - 1;
-            T wv = up ? (s2 >= 1 ? w3[s2 - 1] : T(0)) : (s2 <= 2 ? w3[s2] : T(0));
-            if (o < -dd[i] || o > dd[i]) wv = T(0);
-            wf[s2] = wv;
-            tf[s2] = C[4 * i] * (q[i] - fma(cb + T(o), g.dx[i], g.mn[i]));  // C(i, i)
+        for (int k = 0; k < 4; ++k) {  // slot k = offset + 1 from the cell
+            const int o = k - 1;
+            T wv = up ? (k >= 1 ? w3[k - 1] : T(0)) : (k <= 2 ? w3[k] : T(0));
+            if (clip && (o < -dd[i] || o > dd[i])) wv = T(0);
+            wf[k] = wv;
+            uf[k] = wv * (ci * (f[i] - T(o)));
         }
-        store4(ra + 4 * i, wf);
-        store4(ra + 12 + 4 * i, tf);
-        axis_weights(f - T(0.5f), wc[i], gu);  // cell-centre nodes: middle node = this cell's centre
+        store4(rec + 8 * i, wf);
+        store4(rec + 8 * i + 4, uf);
+        const T m = f[i] - T(0.5f);
+        axis_weights(m, w3, gu);  // cell-centre nodes: middle node = this cell's centre
 #pragma unroll
-        for (int s2 = 0; s2 < 3; ++s2) {
-            const int o = s2 - 1;
-            if (o < -dd[i] || o > dd[i]) wc[i][s2] = T(0);
-            const T dc = q[i] - fma(cb + T(o) + T(0.5f), g.dx[i], g.mn[i]);
+        for (int k = 0; k < 3; ++k) {
+            const int o = k - 1;
+            if (clip && (o < -dd[i] || o > dd[i])) w3[k] = T(0);
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a == i) continue;
                 int b, c;
                 p2g_other_axes(a, b, c);
-                tc[a][b == i ? 0 : 1][s2] = C[3 * a + i] * dc;
+                const T t = (s.C[3 * a + i] * g.dx[i]) * (m - T(o));
+                pair[a][(b == i ? 6 : 0) + 2 * k] = w3[k];
+                pair[a][(b == i ? 6 : 0) + 2 * k + 1] = b == i ? s.v[a] + t : t;
             }
         }
     }
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int b, c;
-        p2g_other_axes(a, b, c);
-        const T va = pv.rest[(3 + a) * cap + ps];
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int s2 = 0; s2 < 3; ++s2)
-#pragma unroll
-            for (int t2 = 0; t2 < 3; ++t2) {
-                const int l = 9 * a + 3 * s2 + t2;
-                rb[l] = wc[b][s2] * wc[c][t2];
-                rb[27 + l] = va + tc[a][0][s2] + tc[a][1][t2];
-            }
-    }
+        for (int k = 0; k < 12; k += 4) store4(rec + 24 + 12 * a + k, pair[a] + k);
     return ci[2] - z0;
 }
 
+// Adds N (weight, value) pairs to the tile's accumulators p[0], p[stride],
+// ...: in single precision both at once by a 64-bit compare-and-swap (a
+// shared-memory float add is a compare-and-swap loop by itself, so a pair
+// costs one loop for two), the first attempts of all pairs in flight
+// together.
+__device__ __forceinline__ unsigned long long p2g_sum(unsigned long long was, float w, float v) {
+    return (unsigned long long)__float_as_uint(__uint_as_float(unsigned(was)) + w) |
+           ((unsigned long long)__float_as_uint(__uint_as_float(unsigned(was >> 32)) + v) << 32);
+}
+template <int N> __device__ __forceinline__ void p2g_add(float2* p, int stride, const float (&w)[N], const float (&v)[N]) {
+    unsigned long long was[N], now[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) was[i] = *reinterpret_cast<volatile unsigned long long*>(p + i * stride);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        now[i] = atomicCAS(reinterpret_cast<unsigned long long*>(p + i * stride), was[i], p2g_sum(was[i], w[i], v[i]));
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        while (now[i] != was[i]) {
+            was[i] = now[i];
+            now[i] = atomicCAS(reinterpret_cast<unsigned long long*>(p + i * stride), was[i],
+                               p2g_sum(was[i], w[i], v[i]));
+        }
+}
+template <int N>
+__device__ __forceinline__ void p2g_add(double2* p, int stride, const double (&w)[N], const double (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        atomicAdd(&p[i * stride].x, w[i]);
+        atomicAdd(&p[i * stride].y, v[i]);
+    }
+}
+
 // LiquidModel<3>::Particle2Grid accumulation (LiquidModel.cpp:614-701).
-// One CTA per 8^3-cell tile, shared-memory accumulators for the tile's
-// window nodes of the three face components.  A warp takes whole z rows of
-// the tile: the particles of a row are contiguous in the sorted order.  The
-// row's particles are staged 16 at a time (one lane per particle computes
-// its per-axis weights and C.(x_p - x_node) terms once, for all three
-// components, and the per-column products below), then the warp walks them
-// run by run (a ballot over the staged cell offsets marks where each cell's
-// particles start), two at a time within a run: lane l < 27 owns one
-// column of 4 window nodes of one component (component l / 9, along that
-// component's own axis; the 3 x 3 columns across it) and sums the weights
-// and APIC values of the current cell's particles in registers.  When the
-// walk reaches the next cell each lane adds its 4 nodes once into the
-// tile's accumulators; at the end every touched node goes to global memory
-// with one add.  The per-axis weights are the reference's B-spline in closed
-// form; the per-node products are regrouped and fused and particles are
-// summed in another order, so P2G matches the reference to rounding, not
-// bit for bit.  No per-particle global atomics.
+// One CTA per 8^3-cell tile, shared-memory accumulators (weight, value) for
+// the tile's window nodes of the three face components.  A warp takes whole
+// z rows of the tile: the particles of a row are contiguous in the sorted
+// order.  The row's particles are staged kP2GChunk at a time (one lane per
+// particle forms its per-axis weights and C.(x_p - x_node) terms once, for
+// all three components), then the warp walks them run by run (a ballot over
+// the staged cell offsets marks where each cell's particles start): lane
+// l < 27 owns one column of 4 window nodes of one component (component l / 9,
+// along that component's own axis; the 3 x 3 columns across it) and sums the
+// weights and APIC values of the current cell's particles in registers, the
+// four nodes as packed pairs.  When the walk reaches the next cell each lane
+// adds its 4 nodes once into the tile's accumulators; at the end every
+// touched node goes to global memory with one add.  The per-axis weights are
+// the reference's B-spline in closed form; the per-node products are
+// regrouped and fused and particles are summed in another order, so P2G
+// matches the reference to rounding, not bit for bit.  No per-particle
+// global atomics.
+// What bounds it: shared-memory wavefronts (23 a particle, 75% of the pipe's
+// rate: a walking lane receives 48 bytes for its 4 nodes, 12 wavefronts a
+// warp whatever the lanes share), then issue (55 instructions a particle).
+// 256^3 dam break, 32.2 M particles: 2.87 ms; 3.08 ms with separate
+// weight and value adds per node and half the lanes staging.
 template <class T>
-__global__ void __launch_bounds__(kP2GWarps * 32, sizeof(T) == 4 ? 3 : 1) k_p2g(GridP<T> g, const int32_t* __restrict__ cs, PView<T> pv,
-                                                        int d0, int d1, int d2, P2GOut<T> out,
-                                                        int* __restrict__ ov_count, int32_t* __restrict__ ov_list) {
+__global__ void __launch_bounds__(kP2GWarps * 32, sizeof(T) == 4 ? 3 : 1)
+    k_p2g(GridP<T> g, const int32_t* __restrict__ cs, PView<T> pv, int d0, int d1, int d2, P2GOut<T> out,
+          int* __restrict__ ov_count, int32_t* __restrict__ ov_list) {
+    using T2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+    using V = Lanes<T, 2>;
+    using P = typename V::P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* acc = reinterpret_cast<T*>(smem_raw);
+    T2* acc = reinterpret_cast<T2*>(smem_raw);
     __shared__ int any;
     const int x0 = blockIdx.z * kTile, y0 = blockIdx.y * kTile, z0 = blockIdx.x * kTile;
     const int zend = min(z0 + kTile, g.nz);
     const int R0 = p2g_region(0), R1 = p2g_region(1), R2 = p2g_region(2);
-    const int ntot = 2 * (R0 + R1 + R2);
-    static_assert(kP2GStage % 4 == 0 && kP2GRecA % 4 == 0, "records stay 16-byte aligned");
-    T* stA = acc + ntot + (threadIdx.x >> 5) * kP2GStage;  // ntot is a multiple of 4
-    T* stB = stA + kP2GChunk * kP2GRecA;
+    const int ntot = R0 + R1 + R2;
+    static_assert((p2g_region(0) + p2g_region(1) + p2g_region(2)) % 2 == 0 && kP2GStage % 4 == 0 && kP2GRec % 4 == 0,
+                  "records stay 16-byte aligned");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T* stage = reinterpret_cast<T*>(acc + ntot) + warp * kP2GStage;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
     if (threadIdx.x < kTile * kTile) {  // row (x0 + t / 8, y0 + t % 8)
@@ -583,65 +617,53 @@ __global__ void __launch_bounds__(kP2GWarps * 32, sizeof(T) == 4 ? 3 : 1) k_p2g(
     }
     __syncthreads();
     if (!any) return;
-    for (int i = threadIdx.x; i < ntot; i += blockDim.x) acc[i] = T(0);
+    for (int i = threadIdx.x; i < ntot; i += blockDim.x) acc[i] = T2{T(0), T(0)};
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // this lane's column: component a, centre slots s (axis b) and t (axis c), face slots k along a
-    const int a = lane / 9, s = (lane % 9) / 3, t = lane % 3;
-    int b = 0, c = 0;
-    p2g_other_axes(a < 3 ? a : 0, b, c);
+    const int dd[3] = {d0, d1, d2};
+    // this lane's column: component a, centre slots sl (axis b) and tl (axis c), face slots along a; lanes
+    // 27-31 walk column 0 and add nothing
     const bool col = lane < 27;
-    const int ac = col ? a : 0;
-    const int ey = kTile + 2 + (ac == 1), ez = kTile + 2 + (ac == 2);
-    const int astride = (ac == 0) ? ey * ez : (ac == 1) ? ez : 1;
+    const int lc = col ? lane : 0;
+    const int a = lc / 9, sl = (lc % 9) / 3, tl = lc % 3;
+    const int ey = kTile + 2 + (a == 1), ez = kTile + 2 + (a == 2);
+    const int astride = (a == 0) ? ey * ez : (a == 1) ? ez : 1;
     // the column's first node relative to its cell, per axis (slot - 1, plus 1 for the halo): face slot 0
-    // along a, centre slot s along b, t along c (b < c)
-    const int ox = (ac == 0) ? 0 : s;
-    const int oy = (ac == 1) ? 0 : (b == 1 ? s : t);
-    const int oz = (ac == 2) ? 0 : t;
-    // component a's weight and value accumulators: [w_0 | v_0 | w_1 | v_1 | w_2 | v_2]
-    T* aw_s = acc + ((ac == 1) ? 2 * R0 : (ac == 2) ? 2 * (R0 + R1) : 0);
-    T* av_s = aw_s + ((ac == 1) ? R1 : (ac == 2) ? R2 : R0);
-    const int lw = col ? lane : 0;  // record offsets of this lane's column
+    // along a, centre slot sl along b, tl along c (b < c)
+    const int ox = (a == 0) ? 0 : sl, oy = (a == 1) ? 0 : (a == 0) ? sl : tl, oz = (a == 2) ? 0 : tl;
+    T2* acc_a = acc + ((a == 1) ? R0 : (a == 2) ? R0 + R1 : 0) + (ox * ey + oy) * ez + oz;
+    const T* rec_f = stage + 8 * a;
+    const T* rec_c = stage + 24 + 12 * a + 2 * tl;
+    const T* rec_b = stage + 30 + 12 * a + 2 * sl;
+    const T zz[2] = {T(0), T(0)};
     for (int row = warp; row < kTile * kTile; row += kP2GWarps) {
         const int rx = x0 + (row >> 3), ry = y0 + (row & 7);
         if (rx >= g.nx || ry >= g.ny) continue;
         const long long c0 = ((long long)rx * g.ny + ry) * g.nz + z0;
         const int pbeg = cs[c0], pend = cs[c0 + (zend - z0)];
         if (pend == pbeg) continue;
+        T2* acc_r = acc_a + ((rx - x0) * ey + (ry - y0)) * ez;
         int cur = -1;  // z offset of the cell being summed
-        T aw[4] = {T(0), T(0), T(0), T(0)}, av[4] = {T(0), T(0), T(0), T(0)};
+        P w0 = V::pack(zz), w1 = w0, v0 = w0, v1 = w0;
         auto flush = [&]() {
-            if (cur < 0 || !col) return;
-            // window node of slot (k, s, t) of cell (rx, ry, z0 + cur), local to the tile region
-            const int base = (((rx - x0) + ox) * ey + (ry - y0) + oy) * ez + cur + oz;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                atomicAdd(&aw_s[base + k * astride], aw[k]);
-                atomicAdd(&av_s[base + k * astride], av[k]);
-                aw[k] = T(0);
-                av[k] = T(0);
+            if (col) {
+                T w[4], v[4];
+                V::unpack(w0, w);
+                V::unpack(w1, w + 2);
+                V::unpack(v0, v);
+                V::unpack(v1, v + 2);
+                p2g_add<4>(acc_r + cur, astride, w, v);
             }
-        };
-        auto add = [&](int j) {
-            T wf[4], tf[4];
-            load4(stA + j * kP2GRecA + 4 * ac, wf);
-            load4(stA + j * kP2GRecA + 12 + 4 * ac, tf);
-            const T W = stB[j * kP2GRecB + lw], B = stB[j * kP2GRecB + 27 + lw];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const T w = W * wf[k];
-                aw[k] += w;
-                av[k] = fma(w, B + tf[k], av[k]);
-            }
+            w0 = w1 = v0 = v1 = V::pack(zz);
         };
         for (int chunk = pbeg; chunk < pend; chunk += kP2GChunk) {
             const int n = min(kP2GChunk, pend - chunk);
             __syncwarp();
-            int zo = -1;  // this lane's particle: z offset of its cell in the row (-1: overflow)
-            if (lane < n)
-                zo = p2g_stage<T>(g, d0, d1, d2, pv, chunk + lane, rx, ry, z0, zend, stA + lane * kP2GRecA,
-                                  stB + lane * kP2GRecB, ov_count, ov_list);
+            int zo = -1;  // this lane's particle: z offset of its cell in the row (-1: listed for k_p2g_overflow)
+            if (lane < n) {
+                P2GParticle<T> part;
+                p2g_fetch(pv, chunk + lane, part);
+                zo = p2g_stage(g, dd, part, chunk + lane, rx, ry, z0, zend, stage + lane * kP2GRec, ov_count, ov_list);
+            }
             __syncwarp();
             // the chunk's runs of particles of one cell (sorted order: a cell's particles are contiguous);
             // every lane walks the same runs
@@ -652,22 +674,30 @@ __global__ void __launch_bounds__(kP2GWarps * 32, sizeof(T) == 4 ? 3 : 1) k_p2g(
                 starts &= starts - 1;
                 const int se = starts ? __ffs(starts) - 1 : n;
                 const int run = __shfl_sync(0xffffffffu, zo, sb);
-                if (run < 0) continue;  // overflow particles: k_p2g_overflow adds them
+                if (run < 0) continue;
                 if (run != cur) {
-                    flush();
+                    if (cur >= 0) flush();
                     cur = run;
                 }
-                if (col) {
-                    int j = sb;
-                    for (; j + 1 < se; j += 2) {
-                        add(j);
-                        add(j + 1);
-                    }
-                    if (j < se) add(j);
+#pragma unroll 2
+                for (int j = sb * kP2GRec; j < se * kP2GRec; j += kP2GRec) {
+                    P wf[2], uf[2];
+                    T c2[2], b2[2];
+                    load_pairs(rec_f + j, wf);
+                    load_pairs(rec_f + j + 4, uf);
+                    load2(rec_c + j, c2);
+                    load2(rec_b + j, b2);
+                    const T W = b2[0] * c2[0], WB = W * (b2[1] + c2[1]);
+                    const T ww[2] = {W, W}, wb[2] = {WB, WB};
+                    const P W2 = V::pack(ww), B2 = V::pack(wb);
+                    w0 = V::fmadd(W2, wf[0], w0);
+                    w1 = V::fmadd(W2, wf[1], w1);
+                    v0 = V::fmadd(B2, wf[0], V::fmadd(W2, uf[0], v0));
+                    v1 = V::fmadd(B2, wf[1], V::fmadd(W2, uf[1], v1));
                 }
             }
         }
-        flush();
+        if (cur >= 0) flush();
     }
     __syncthreads();
     // flush: one global add per touched node
@@ -675,19 +705,18 @@ __global__ void __launch_bounds__(kP2GWarps * 32, sizeof(T) == 4 ? 3 : 1) k_p2g(
     for (int a2 = 0; a2 < 3; ++a2) {
         const int fy2 = kTile + 2 + (a2 == 1), fz2 = kTile + 2 + (a2 == 2);
         const int R = (a2 == 0) ? R0 : (a2 == 1) ? R1 : R2;
-        const T* sw_a = acc + ((a2 == 1) ? 2 * R0 : (a2 == 2) ? 2 * (R0 + R1) : 0);
-        const T* sv_a = sw_a + R;
+        const T2* s_a = acc + ((a2 == 1) ? R0 : (a2 == 2) ? R0 + R1 : 0);
         const int fy = g.ny + (a2 == 1), fz = g.nz + (a2 == 2);
         const int hx = g.nx - 1 + (a2 == 0);
         for (int i = threadIdx.x; i < R; i += blockDim.x) {
-            T wv = sw_a[i], vv = sv_a[i];
-            if (wv == T(0) && vv == T(0)) continue;
+            const T2 wv = s_a[i];
+            if (wv.x == T(0) && wv.y == T(0)) continue;
             int lz = i % fz2, ly = (i / fz2) % fy2, lx = i / (fy2 * fz2);
             int xi = x0 - 1 + lx, yi = y0 - 1 + ly, zi = z0 - 1 + lz;
             if (xi < 0 || xi > hx || yi < 0 || yi >= fy || zi < 0 || zi >= fz) continue;
             long long gi = ((long long)xi * fy + yi) * fz + zi;
-            atomicAdd(&out.w[a2][gi], wv);
-            atomicAdd(&out.v[a2][gi], vv);
+            atomicAdd(&out.w[a2][gi], wv.x);
+            atomicAdd(&out.v[a2][gi], wv.y);
         }
     }
 }

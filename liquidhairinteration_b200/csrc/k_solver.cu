@@ -641,13 +641,15 @@ __device__ __forceinline__ bool rb_eval(const float* __restrict__ Zs, const floa
 }
 
 // Tile id u of the active list -> origin of its 8 x 8 x 32 cells.
-__device__ __forceinline__ void tile_origin(const int32_t* __restrict__ ids, int u, int tdy, int tdz, int& x0, int& y0,
-                                            int& z0) {
-    const int id = ids[u];
+__device__ __forceinline__ void tile_origin_of(int id, int tdy, int tdz, int& x0, int& y0, int& z0) {
     const int tz = id % tdz, rest = id / tdz;
     z0 = tz * kTileZ;
     y0 = (rest % tdy) * kTileY;
     x0 = (rest / tdy) * kTileX;
+}
+__device__ __forceinline__ void tile_origin(const int32_t* __restrict__ ids, int u, int tdy, int tdz, int& x0, int& y0,
+                                            int& z0) {
+    tile_origin_of(ids[u], tdy, tdz, x0, y0, z0);
 }
 
 __device__ __forceinline__ void rb_issue(unsigned char* st, uint64_t* bar, const CUtensorMap* mz, const CUtensorMap* mr,
@@ -674,21 +676,30 @@ __global__ void __launch_bounds__(rb::kThreads, 1)
                const int* __restrict__ count, int tdy, int tdz, float* __restrict__ zout, float w, int variant,
                SolveScalars* __restrict__ sc, const float* __restrict__ ap, double* __restrict__ partials,
                unsigned* __restrict__ counter, int final_dot, int region, int flexible) {
-    if (sc->stop) return;
     extern __shared__ __align__(128) unsigned char sm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
     double v[2] = {0.0, 0.0};  // r.z and Ap.z of the swept tiles (final_dot)
+    // the loads that lead to the first copy, all at once (the list has at
+    // least gridDim.x entries whatever the count), and the maps' descriptors
+    const int stop = sc->stop, units = *count, id0 = ids[blockIdx.x];
     if (threadIdx.x == 0) {
+        prefetch_map(&mz);
+        prefetch_map(&mr);
+        prefetch_map(&md);
+        prefetch_map(&mcx);
+        prefetch_map(&mcy);
+        prefetch_map(&mcz);
+        prefetch_map(&mm);
         bar_init(&bar[0], 1);
         bar_init(&bar[1], 1);
     }
-    __syncthreads();
-    const int units = *count;
+    if (stop) return;
     if (threadIdx.x == 0 && int(blockIdx.x) < units) {
         int a, b, c;
-        tile_origin(ids, blockIdx.x, tdy, tdz, a, b, c);
+        tile_origin_of(id0, tdy, tdz, a, b, c);
         rb_issue(sm + rb::kBase, &bar[0], &mz, &mr, &md, &mcx, &mcy, &mcz, &mm, a, b, c);
     }
+    __syncthreads();
     int it = 0;
     for (int u = blockIdx.x; u < units; u += gridDim.x, ++it) {
         const int s = it & 1;
@@ -1049,46 +1060,7 @@ __global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, Cluste
     reinterpret_cast<uint32_t*>(row + size_t(cl::kVecs<T>) * C.items * 16)[q] = m;
 }
 
-// A thread's slots in groups of W: one value, or two floats in one 64-bit
-// register pair for the packed instructions (each half rounded as the scalar
-// instruction rounds it).
-template <class T, int W> struct Lanes;
-template <class T> struct Lanes<T, 1> {
-    using P = T;
-    static __device__ __forceinline__ P pack(const T* v) { return v[0]; }
-    static __device__ __forceinline__ void unpack(P p, T* v) { v[0] = p; }
-    static __device__ __forceinline__ P mul(P a, P b) { return X<T>::mul(a, b); }
-    static __device__ __forceinline__ P add(P a, P b) { return X<T>::add(a, b); }
-    static __device__ __forceinline__ P fmadd(P a, P b, P c) { return fma(a, b, c); }
-};
-template <> struct Lanes<float, 2> {
-    using P = unsigned long long;
-    static __device__ __forceinline__ P pack(const float* v) {
-        P p;
-        asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(v[0]), "f"(v[1]));
-        return p;
-    }
-    static __device__ __forceinline__ void unpack(P p, float* v) {
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
-    }
-    static __device__ __forceinline__ P mul(P a, P b) {
-        P r;
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-        return r;
-    }
-    static __device__ __forceinline__ P add(P a, P b) {
-        P r;
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-        return r;
-    }
-    static __device__ __forceinline__ P fmadd(P a, P b, P c) {
-        P r;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-        return r;
-    }
-};
-
-// The division of the rare operands (see cluster_term).
+// The division of the rare operands (see ClusterSlots::term).
 template <class T> __device__ __noinline__ T cluster_div(T n, T d) { return X<T>::div(n, d); }
 
 // Rows of a thread's slots: NK of each colour, in groups of W.

@@ -74,6 +74,11 @@ __device__ __forceinline__ void tma_load_box(void* dst, const CUtensorMap* map, 
         : "memory");
 }
 
+// Brings a tensor map's descriptor into the cache its copies read it from.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
 // 4D box load at element coordinates (c0 innermost .. c3) into dst.
 __device__ __forceinline__ void tma_load_box4(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                               uint64_t* bar) {
