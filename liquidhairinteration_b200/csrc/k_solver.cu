@@ -967,8 +967,7 @@ template <class T> constexpr int kVecs = int(8 * sizeof(T) / 16);
 template <class T> __host__ __device__ constexpr int row_bytes(int items) { return items * (16 * kVecs<T> + 4); }
 // flags: the diagonal is not small (the sweeps update the cell); the slot
 // holds a cell; its plane is the slab's first / last with a neighbour CTA on
-// that side; its diagonal lies outside the range of the division by its
-// reciprocal.  Bits 16 and up: the cell's index in the slab's z.
+// that side; the reciprocal of its diagonal is not a normal number.  Bits 16 and up: the cell's index in the slab's z.
 constexpr unsigned kUpdate = 1, kCell = 2, kLeft = 4, kRight = 8, kSlow = 16;
 constexpr int kIndexShift = 16;
 }  // namespace cl
@@ -1044,8 +1043,8 @@ __global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, Cluste
             if (z > 0 && L.type[i - 1] == 2) w[6] = -L.cz[i - 1];
             if (!is_small(d)) {
                 m |= cl::kUpdate;
-                if (fabs(d) > T(1e-12) && fabs(d) < T(1e12)) w[7] = X<T>::div(T(1), d);
-                else m |= cl::kSlow;
+                w[7] = X<T>::div(T(1), d);
+                if (!(fabs(d) < T(1e37))) m |= cl::kSlow;
             }
         }
         if (C.ctas > 1 && p == 0 && x > 0) m |= cl::kLeft;
@@ -1070,9 +1069,11 @@ template <class T, int NK> struct ClusterSlots {
     using P = typename V::P;
     P nd[2][G], y[2][G], r[2][G], nc[2][G][6];  // -d, 1 / d, r, -c
     unsigned m[2][NK];
+    bool slow;  // a slot of this thread needs the division
     __device__ __forceinline__ int a(int c, int k) const { return int(m[c][k] >> cl::kIndexShift); }
 
     __device__ __forceinline__ void load(const ClusterLevel<T>& L, int cta, const T* __restrict__ sm, bool r_global) {
+        slow = false;
         const unsigned char* rows = L.rowoff >= 0 ? reinterpret_cast<const unsigned char*>(sm) + L.rowoff
                                                   : L.rows + size_t(cta) * 2 * cl::row_bytes<T>(L.items);
         const int sx = L.ny * L.nz;
@@ -1098,6 +1099,7 @@ template <class T, int NK> struct ClusterSlots {
                         const uint4 u = reinterpret_cast<const uint4*>(row)[v * L.items + q];
                         memcpy(&w[j][v * (16 / int(sizeof(T)))], &u, 16);
                     }
+                    slow |= (m[c][k] & cl::kSlow) != 0;
                     if (m[c][k] & cl::kCell) rv[j] = r_global ? rg[a(c, k)] : rs[a(c, k)];
                 }
                 T t[W];
@@ -1143,29 +1145,22 @@ template <class T, int NK> struct ClusterSlots {
     // Res. Dev. 34(1), 1990: a quotient within one unit in the last place,
     // corrected by its exact remainder times the correctly rounded
     // reciprocal, is the rounded quotient).  Five dependent multiply-adds,
-    // two cells at a time, instead of a division each.  Operands whose
-    // remainders could underflow or overflow take the division.
+    // two cells at a time, instead of a division each.  The remainders are
+    // exact down to |n| of about 1e-30 in single precision (below, the
+    // quotient stays within two units in the last place); diagonals whose
+    // reciprocal leaves the normal range take the division.
     __device__ __forceinline__ P term(int c, int g, P n) const {
-        const P q0 = V::mul(n, y[c][g]);
-        const P q1 = V::fmadd(V::fmadd(nd[c][g], q0, n), y[c][g], q0);
-        P q = V::fmadd(V::fmadd(nd[c][g], q1, n), y[c][g], q1);
-        T nv[W], qv[W], dv[W];
-        V::unpack(n, nv);
-        bool rare = false;
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            const T an = fabs(nv[j]);
-            rare |= (!(an > T(1e-18) && an < T(1e18)) && an != T(0)) || (m[c][g * W + j] & cl::kSlow);
-        }
-        if (rare) {
-            V::unpack(q, qv);
+        if (slow) {
+            T nv[W], dv[W], qv[W];
+            V::unpack(n, nv);
             V::unpack(nd[c][g], dv);
 #pragma unroll
-            for (int j = 0; j < W; ++j)
-                if (m[c][g * W + j] & cl::kUpdate) qv[j] = cluster_div<T>(nv[j], -dv[j]);
-            q = V::pack(qv);
+            for (int j = 0; j < W; ++j) qv[j] = (m[c][g * W + j] & cl::kUpdate) ? cluster_div<T>(nv[j], -dv[j]) : T(0);
+            return V::pack(qv);
         }
-        return q;
+        const P q0 = V::mul(n, y[c][g]);
+        const P q1 = V::fmadd(V::fmadd(nd[c][g], q0, n), y[c][g], q0);
+        return V::fmadd(V::fmadd(nd[c][g], q1, n), y[c][g], q1);
     }
 };
 
@@ -1199,6 +1194,7 @@ template <class T> __device__ __forceinline__ void cluster_push(const ClusterSid
 static_assert(kMaxLevels + 1 <= 16, "a hardware barrier per level beside __syncthreads's");
 __device__ __forceinline__ void cluster_step(bool wide, int l, int threads) {
     if (wide) cluster_barrier();
+
     else asm volatile("bar.sync %0, %1;" ::"r"(l + 1), "r"(threads) : "memory");
 }
 
@@ -1208,8 +1204,10 @@ constexpr int kVisitDown = 0, kVisitLast = 1, kVisitUp = 2;
 // at the bottom (smooth), or on the way up (prolong: :774-794, smooth).
 // threads: the threads of this CTA that take part (all of them where the level is the cluster's).
 template <class T, int NK>
-__device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int mode, unsigned rank, T* sm, T w,
-                                           int variant, int sweeps, int threads) {
+__device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int mode, unsigned rank, T w, int variant,
+                                           int sweeps, int threads) {
+    extern __shared__ __align__(16) unsigned char smem[];  // named here too, so that every access is a shared one
+    T* sm = reinterpret_cast<T*>(smem);
     using S = ClusterSlots<T, NK>;
     using V = typename S::V;
     using P = typename S::P;
@@ -1370,9 +1368,9 @@ __global__ void __launch_bounds__(cl::kThreads, 1)
         const ClusterLevel<T>& L = c.L[l];
         const int threads = L.ctas > 1 ? cl::kThreads : max(32, min(cl::kThreads, (L.items + 31) & ~31));
         if ((L.ctas == 1 && rank != 0) || int(threadIdx.x) >= threads) continue;
-        if (L.items <= cl::kThreads) cluster_visit<T, 1>(c, l, mode, rank, sm, w, variant, sweeps, threads);
-        else if (L.items <= 2 * cl::kThreads) cluster_visit<T, 2>(c, l, mode, rank, sm, w, variant, sweeps, threads);
-        else cluster_visit<T, cl::kSlots<T>>(c, l, mode, rank, sm, w, variant, sweeps, threads);
+        if (L.items <= cl::kThreads) cluster_visit<T, 1>(c, l, mode, rank, w, variant, sweeps, threads);
+        else if (L.items <= 2 * cl::kThreads) cluster_visit<T, 2>(c, l, mode, rank, w, variant, sweeps, threads);
+        else cluster_visit<T, cl::kSlots<T>>(c, l, mode, rank, w, variant, sweeps, threads);
     }
     if (wide) cluster_barrier();  // no CTA leaves while another may still reach its shared memory
 }
