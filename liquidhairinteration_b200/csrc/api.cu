@@ -16,9 +16,52 @@ struct lhi_liquid {
     std::unique_ptr<lhi::LiquidBase> impl;
 };
 
+// Device copies of the host buffers of the network entry points, kept by the
+// network for its next call (allocating and freeing them took most of a call:
+// cudaFree waits for the device) and sized by the largest grid so far.
+struct NetStaging {
+    float* r = nullptr;
+    uint8_t* type = nullptr;
+    uint8_t* solid = nullptr;
+    float* z = nullptr;
+    float* dz = nullptr;
+    long long cap = 0, cap_dz = 0;
+    void release() {
+        cudaFree(r);
+        cudaFree(type);
+        cudaFree(solid);
+        cudaFree(z);
+        r = z = nullptr;
+        type = solid = nullptr;
+        cap = 0;
+    }
+    void reserve(long long n, bool grad) {
+        if (n > cap) {
+            release();
+            LHI_CUDA(cudaMalloc(&r, sizeof(float) * n));
+            LHI_CUDA(cudaMalloc(&type, size_t(n)));
+            LHI_CUDA(cudaMalloc(&solid, size_t(n)));
+            LHI_CUDA(cudaMalloc(&z, sizeof(float) * n));
+            cap = n;
+        }
+        if (grad && n > cap_dz) {
+            cudaFree(dz);
+            dz = nullptr;
+            cap_dz = 0;
+            LHI_CUDA(cudaMalloc(&dz, sizeof(float) * n));
+            cap_dz = n;
+        }
+    }
+    ~NetStaging() {
+        release();
+        cudaFree(dz);
+    }
+};
+
 struct lhi_net {
     std::unique_ptr<lhi::LearnedNet> impl;
     cudaStream_t stream = nullptr;
+    NetStaging staging;
     ~lhi_net() {
         impl.reset();
         if (stream) cudaStreamDestroy(stream);
@@ -365,22 +408,6 @@ LHI_API int lhi_net_set_params(lhi_net* net, const float* in) {
 }
 
 namespace {
-// device copies of host inputs for the host-buffer network entry points
-struct NetHostArgs {
-    float* r = nullptr;
-    uint8_t* type = nullptr;
-    uint8_t* solid = nullptr;
-    float* z = nullptr;
-    float* dz = nullptr;
-    ~NetHostArgs() {
-        cudaFree(r);
-        cudaFree(type);
-        cudaFree(solid);
-        cudaFree(z);
-        cudaFree(dz);
-    }
-};
-
 long long net_dims_check(const int32_t dims[3]) {
     if (!dims) throw std::invalid_argument("null dims");
     for (int a = 0; a < 3; ++a)
@@ -388,16 +415,13 @@ long long net_dims_check(const int32_t dims[3]) {
     return (long long)dims[0] * dims[1] * dims[2];
 }
 
-void net_upload(NetHostArgs& d, long long n, const float* r, const uint8_t* type, const uint8_t* solid, cudaStream_t s) {
-    LHI_CUDA(cudaMalloc(&d.r, sizeof(float) * n));
-    LHI_CUDA(cudaMalloc(&d.type, size_t(n)));
-    LHI_CUDA(cudaMalloc(&d.z, sizeof(float) * n));
+void net_upload(NetStaging& d, long long n, const float* r, const uint8_t* type, const uint8_t* solid, const float* dz,
+                cudaStream_t s) {
+    d.reserve(n, dz != nullptr);
     LHI_CUDA(cudaMemcpyAsync(d.r, r, sizeof(float) * n, cudaMemcpyHostToDevice, s));
     LHI_CUDA(cudaMemcpyAsync(d.type, type, size_t(n), cudaMemcpyHostToDevice, s));
-    if (solid) {
-        LHI_CUDA(cudaMalloc(&d.solid, size_t(n)));
-        LHI_CUDA(cudaMemcpyAsync(d.solid, solid, size_t(n), cudaMemcpyHostToDevice, s));
-    }
+    if (solid) LHI_CUDA(cudaMemcpyAsync(d.solid, solid, size_t(n), cudaMemcpyHostToDevice, s));
+    if (dz) LHI_CUDA(cudaMemcpyAsync(d.dz, dz, sizeof(float) * n, cudaMemcpyHostToDevice, s));
 }
 }  // namespace
 
@@ -467,11 +491,11 @@ LHI_API int lhi_net_forward_host(lhi_net* net, const int32_t dims[3], const floa
     if (!net || !r || !type || !z) return fail(LHI_E_INVALID_ARG, "null argument");
     return guarded([&]() -> int {
         const long long n = net_dims_check(dims);
-        NetHostArgs d;
-        net_upload(d, n, r, type, solid, net->stream);
+        NetStaging& d = net->staging;
+        net_upload(d, n, r, type, solid, nullptr, net->stream);
         const int dd[3] = {dims[0], dims[1], dims[2]};
         if (net->impl->sparse_enabled_) net->impl->plan_sparse(dd, d.type, net->stream);
-        net->impl->forward(dd, d.r, d.type, d.solid, d.z, scale, net->stream, true);
+        net->impl->forward(dd, d.r, d.type, solid ? d.solid : nullptr, d.z, scale, net->stream, true);
         LHI_CUDA(cudaMemcpyAsync(z, d.z, sizeof(float) * n, cudaMemcpyDeviceToHost, net->stream));
         LHI_CUDA(cudaStreamSynchronize(net->stream));
         const int st = net->impl->check_status(net->stream);
@@ -488,13 +512,11 @@ LHI_API int lhi_net_backward_host(lhi_net* net, const int32_t dims[3], const flo
     if (!net || !r || !type || !dz || !grad) return fail(LHI_E_INVALID_ARG, "null argument");
     return guarded([&]() -> int {
         const long long n = net_dims_check(dims);
-        NetHostArgs d;
-        net_upload(d, n, r, type, solid, net->stream);
-        LHI_CUDA(cudaMalloc(&d.dz, sizeof(float) * n));
-        LHI_CUDA(cudaMemcpyAsync(d.dz, dz, sizeof(float) * n, cudaMemcpyHostToDevice, net->stream));
+        NetStaging& d = net->staging;
+        net_upload(d, n, r, type, solid, dz, net->stream);
         const int dd[3] = {dims[0], dims[1], dims[2]};
         net->impl->zero_grad(net->stream);
-        net->impl->forward(dd, d.r, d.type, d.solid, d.z, scale, net->stream);
+        net->impl->forward(dd, d.r, d.type, solid ? d.solid : nullptr, d.z, scale, net->stream);
         net->impl->backward(d.dz, net->stream);
         net->impl->get_grads(grad, net->stream);
         const int st = net->impl->check_status(net->stream);
