@@ -876,18 +876,36 @@ template <class T> __device__ void solid_grad_at(const GridP<T>& g, const T* sp,
 // v = sum wX A, C = (sum gX A, sum wX B, sum wX D) -- with fused
 // multiply-adds: about a third of the arithmetic, the same value up to
 // rounding.
-// Where a gather reads the face velocities of one component: the global
-// array (origin 0, the face grid's extents) or a tile's staged copy in
-// shared memory (origin one node before the tile, the region's extents).
-template <class T> struct VSrc {
-    const T* v;
+// Where a gather reads the face velocities: the global arrays, or a tile's
+// staged copy in shared memory (origin one node before the tile), whose
+// strides are constants and whose addresses are plain 32-bit sums.  (One
+// struct with run-time strides for both made every load a generic one behind
+// 64-bit multiplies.)
+template <class T> struct GlobalSrc {
+    const T* v[3];
+    int ny, nz;
+    template <int A> __device__ __forceinline__ const T* at(int x, int y, int z) const {
+        return v[A] + ((long long)x * (ny + (A == 1)) + y) * (nz + (A == 2)) + z;
+    }
+};
+template <class T> struct StagedSrc {
+    const T* sv;
     int ox, oy, oz;
-    long long fy, fz;
+    template <int A> __device__ __forceinline__ const T* at(int x, int y, int z) const {
+        constexpr int off = (A == 0) ? 0 : p2g_region(0) + (A == 2 ? p2g_region(1) : 0);
+        constexpr int fy = kTile + 2 + (A == 1), fz = kTile + 2 + (A == 2);
+        return sv + off + ((x - ox) * fy + (y - oy)) * fz + (z - oz);
+    }
 };
 
-template <class T, int A, bool FACTORED>
+// A particle's velocity and affine matrix, as gathered.
+template <class T> struct G2pSum {
+    T vel[3], C[9];
+};
+
+template <class T, int A, bool FACTORED, class Src>
 __device__ __forceinline__ void g2p_component(const GridP<T>& g, const int d[3], const T g3[3], const int ci[3],
-                                              const VSrc<T> vs, T& velA, T col[3]) {
+                                              const Src& vs, T& velA, T col[3]) {
     const int hmax[3] = {g.nx - 1 + (A == 0), g.ny - 1 + (A == 1), g.nz - 1 + (A == 2)};
     T ew[3][3], eg[3][3];
     int first[3], cnt[3];
@@ -925,8 +943,7 @@ __device__ __forceinline__ void g2p_component(const GridP<T>& g, const int d[3],
 #pragma unroll
             for (int jy = 0; jy < 3; ++jy) {
                 if (jy >= cnt[1]) break;
-                const T* row = vs.v + ((long long)(first[0] + jx - vs.ox) * vs.fy + (first[1] + jy - vs.oy)) * vs.fz +
-                               (first[2] - vs.oz);
+                const T* row = vs.template at<A>(first[0] + jx, first[1] + jy, first[2]);
                 T s = T(0), t = T(0);
 #pragma unroll
                 for (int jz = 0; jz < 3; ++jz) {
@@ -954,8 +971,7 @@ __device__ __forceinline__ void g2p_component(const GridP<T>& g, const int d[3],
             if (jy >= cnt[1]) break;
             const T wY = ew[1][jy], gY = eg[1][jy];
             const T wXY = X<T>::mul(wX, wY), gXwY = X<T>::mul(gX, wY), wXgY = X<T>::mul(wX, gY);
-            const T* row = vs.v + ((long long)(first[0] + jx - vs.ox) * vs.fy + (first[1] + jy - vs.oy)) * vs.fz +
-                               (first[2] - vs.oz);
+            const T* row = vs.template at<A>(first[0] + jx, first[1] + jy, first[2]);
 #pragma unroll
             for (int jz = 0; jz < 3; ++jz) {
                 if (jz >= cnt[2]) break;
@@ -989,7 +1005,7 @@ __device__ __forceinline__ void g2p_component(const GridP<T>& g, const int d[3],
 template <class T, int A>
 __device__ __forceinline__ void g2p_staged_component(const T wf[3][3], const T gf[3][3], const T wc[3][3],
                                                      const T gc[3][3], const int mf[3], const int ci[3],
-                                                     const VSrc<T>& vs, T& velA, T col[3]) {
+                                                     const StagedSrc<T>& vs, T& velA, T col[3]) {
     const int bx = ((A == 0) ? mf[0] : ci[0]) - 1, by = ((A == 1) ? mf[1] : ci[1]) - 1,
               bz = ((A == 2) ? mf[2] : ci[2]) - 1;
     const T* wx = (A == 0) ? wf[0] : wc[0];
@@ -998,13 +1014,14 @@ __device__ __forceinline__ void g2p_staged_component(const T wf[3][3], const T g
     const T* gy = (A == 1) ? gf[1] : gc[1];
     const T* wz = (A == 2) ? wf[2] : wc[2];
     const T* gz = (A == 2) ? gf[2] : gc[2];
-    const T* base = vs.v + ((long long)(bx - vs.ox) * vs.fy + (by - vs.oy)) * vs.fz + (bz - vs.oz);
+    const T* base = vs.template at<A>(bx, by, bz);
+    constexpr int fy = kTile + 2 + (A == 1), fz = kTile + 2 + (A == 2);
 #pragma unroll
     for (int jx = 0; jx < 3; ++jx) {
         T a = T(0), b = T(0), dd = T(0);
 #pragma unroll
         for (int jy = 0; jy < 3; ++jy) {
-            const T* row = base + ((long long)jx * vs.fy + jy) * vs.fz;
+            const T* row = base + (jx * fy + jy) * fz;
             T s = T(0), t = T(0);
 #pragma unroll
             for (int jz = 0; jz < 3; ++jz) {
@@ -1024,8 +1041,8 @@ __device__ __forceinline__ void g2p_staged_component(const T wf[3][3], const T g
 }
 
 template <class T>
-__device__ __forceinline__ void g2p_staged_factored(const GridP<T>& g, const int d[3], const T g3[3], const int ci[3],
-                                                    const VSrc<T> src[3], T vel[3], T C[9]) {
+__device__ __forceinline__ void g2p_staged_factored(const T g3[3], const int ci[3], const StagedSrc<T>& vs,
+                                                    G2pSum<T>& r) {
     T wf[3][3], gf[3][3], wc[3][3], gc[3][3];
     int mf[3];
 #pragma unroll
@@ -1036,34 +1053,46 @@ __device__ __forceinline__ void g2p_staged_factored(const GridP<T>& g, const int
         axis_weights(g3[i] - T(mf[i]), wf[i], gf[i]);
         axis_weights(f - T(0.5f), wc[i], gc[i]);
     }
-    g2p_staged_component<T, 0>(wf, gf, wc, gc, mf, ci, src[0], vel[0], &C[0]);
-    g2p_staged_component<T, 1>(wf, gf, wc, gc, mf, ci, src[1], vel[1], &C[3]);
-    g2p_staged_component<T, 2>(wf, gf, wc, gc, mf, ci, src[2], vel[2], &C[6]);
+    g2p_staged_component<T, 0>(wf, gf, wc, gc, mf, ci, vs, r.vel[0], &r.C[0]);
+    g2p_staged_component<T, 1>(wf, gf, wc, gc, mf, ci, vs, r.vel[1], &r.C[3]);
+    g2p_staged_component<T, 2>(wf, gf, wc, gc, mf, ci, vs, r.vel[2], &r.C[6]);
 }
 
-// The factored gather of the particles the staged closed-form path does not
-// take (near the grid's faces, off the tile, or a window below +-2), kept
-// out of line so that its registers do not weigh on the common path.
-template <class T>
-__device__ __noinline__ void g2p_general_factored(const GridP<T>& g, const int d[3], const T g3[3], const int ci[3],
-                                                  const VSrc<T> src[3], T vel[3], T C[9]) {
-    g2p_component<T, 0, true>(g, d, g3, ci, src[0], vel[0], &C[0]);
-    g2p_component<T, 1, true>(g, d, g3, ci, src[1], vel[1], &C[3]);
-    g2p_component<T, 2, true>(g, d, g3, ci, src[2], vel[2], &C[6]);
+// The general gather of one particle.
+template <class T, bool FACTORED, class Src>
+__device__ __forceinline__ void g2p_components(const GridP<T>& g, const int d[3], const T g3[3], const int ci[3],
+                                               const Src& src, G2pSum<T>& r) {
+    g2p_component<T, 0, FACTORED>(g, d, g3, ci, src, r.vel[0], &r.C[0]);
+    g2p_component<T, 1, FACTORED>(g, d, g3, ci, src, r.vel[1], &r.C[3]);
+    g2p_component<T, 2, FACTORED>(g, d, g3, ci, src, r.vel[2], &r.C[6]);
+}
+
+// The same out of line, for the particles that the tile kernel's own path does
+// not take (off the tile, and for the factored sums near the grid's faces or
+// with a window below +-2), so that its registers do not weigh on the common
+// path; operands and result go by value so that none of the common path's
+// has an address.
+template <class T, bool FACTORED>
+__device__ __noinline__ G2pSum<T> g2p_general(const GridP<T>& g, int d0, int d1, int d2, T gx, T gy, T gz, int cx,
+                                              int cy, int cz, GlobalSrc<T> src) {
+    const int d[3] = {d0, d1, d2}, ci[3] = {cx, cy, cz};
+    const T g3[3] = {gx, gy, gz};
+    G2pSum<T> r = {};
+    g2p_components<T, FACTORED>(g, d, g3, ci, src, r);
+    return r;
 }
 
 // One particle of LiquidModel<3>::Grid2Particle (LiquidModel.cpp:724-823)
 // fused with AdvectParticle (LiquidModel.cpp:913-935) and the next step's
-// cell key.  The face velocities come from the sources the caller picks
-// for the particle's truncated cell ci (staged in shared memory when ci lies
-// in the tile -- pick returns true -- global memory otherwise).
-template <class T, bool FACTORED, class PickSrc>
+// cell key.  The face velocities come from the tile's staged copy (TILE) when
+// the particle's truncated cell ci lies in the tile, from global memory
+// otherwise.
+template <class T, bool FACTORED, bool TILE>
 __device__ __forceinline__ void g2p_particle(const GridP<T>& g, T* __restrict__ pd, long long cap, long long i,
-                                             const int d[3], int do_g2p, int do_advect, T dt,
+                                             T q[3], const int d[3], int do_g2p, int do_advect, T dt,
                                              const T* __restrict__ sp, uint32_t* __restrict__ keys,
-                                             int32_t* __restrict__ vals, PickSrc pick) {
-    T q[3] = {pd[i], pd[cap + i], pd[2 * cap + i]};  // (the positions are rows 0-2 of pd also while the sort's
-                                                     // permutation waits: pd is then the sorted buffer)
+                                             int32_t* __restrict__ vals, const GlobalSrc<T>& src,
+                                             const StagedSrc<T>& tile, int zend) {
     T vel[3];
     if (do_g2p) {
         T g3[3];
@@ -1074,29 +1103,31 @@ __device__ __forceinline__ void g2p_particle(const GridP<T>& g, T* __restrict__ 
             g3[k] = FACTORED ? (q[k] - g.mn[k]) * g.idx[k] : X<T>::div(X<T>::sub(q[k], g.mn[k]), g.dx[k]);
             ci[k] = int(g3[k]);
         }
-        T C[9];
-        vel[0] = vel[1] = vel[2] = T(0);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) C[k] = T(0);
-        VSrc<T> src[3];
-        const bool staged = pick(ci, src);
-        // the staged closed-form path: ci >= 1 (so g3 >= 0 and ci is the floor) and ci <= n - 2 on every
-        // axis with a window of +-2 or more; anything else takes the general path
-        const bool full = d[0] >= 2 && d[1] >= 2 && d[2] >= 2 && ci[0] >= 1 && ci[0] <= g.nx - 2 && ci[1] >= 1 &&
-                          ci[1] <= g.ny - 2 && ci[2] >= 1 && ci[2] <= g.nz - 2;
-        if (FACTORED && staged && full) {
-            g2p_staged_factored<T>(g, d, g3, ci, src, vel, C);
-        } else if constexpr (FACTORED) {
-            g2p_general_factored<T>(g, d, g3, ci, src, vel, C);  // out of line: the rare particles
+        G2pSum<T> r = {};
+        if constexpr (TILE) {
+            // (a particle off the grid is sorted into a clamped cell)
+            bool own = ci[0] > tile.ox && ci[0] <= tile.ox + kTile && ci[1] > tile.oy && ci[1] <= tile.oy + kTile &&
+                       ci[2] > tile.oz && ci[2] < zend;
+            // the closed form: ci >= 1 (so g3 >= 0 and ci is the floor) and ci <= n - 2 on every axis with a
+            // window of +-2 or more
+            if (FACTORED)
+                own = own && d[0] >= 2 && d[1] >= 2 && d[2] >= 2 && ci[0] >= 1 && ci[0] <= g.nx - 2 && ci[1] >= 1 &&
+                      ci[1] <= g.ny - 2 && ci[2] >= 1 && ci[2] <= g.nz - 2;
+            if (!own)
+                r = g2p_general<T, FACTORED>(g, d[0], d[1], d[2], g3[0], g3[1], g3[2], ci[0], ci[1], ci[2], src);
+            else if constexpr (FACTORED)
+                g2p_staged_factored<T>(g3, ci, tile, r);
+            else
+                g2p_components<T, FACTORED>(g, d, g3, ci, tile, r);
         } else {
-            g2p_component<T, 0, FACTORED>(g, d, g3, ci, src[0], vel[0], &C[0]);
-            g2p_component<T, 1, FACTORED>(g, d, g3, ci, src[1], vel[1], &C[3]);
-            g2p_component<T, 2, FACTORED>(g, d, g3, ci, src[2], vel[2], &C[6]);
+            g2p_components<T, FACTORED>(g, d, g3, ci, src, r);
         }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) vel[k] = r.vel[k];
 #pragma unroll
         for (int k = 0; k < 3; ++k) pd[(3 + k) * cap + i] = vel[k];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) pd[(6 + k) * cap + i] = C[k];
+        for (int k = 0; k < 9; ++k) pd[(6 + k) * cap + i] = r.C[k];
     } else {
 #pragma unroll
         for (int k = 0; k < 3; ++k) vel[k] = pd[(3 + k) * cap + i];
@@ -1123,13 +1154,6 @@ __device__ __forceinline__ void g2p_particle(const GridP<T>& g, T* __restrict__ 
     }
 }
 
-template <class T> __device__ __forceinline__ void global_sources(const GridP<T>& g, const T* vx, const T* vy,
-                                                                  const T* vz, VSrc<T> src[3]) {
-    src[0] = VSrc<T>{vx, 0, 0, 0, g.ny, g.nz};
-    src[1] = VSrc<T>{vy, 0, 0, 0, g.ny + 1, g.nz};
-    src[2] = VSrc<T>{vz, 0, 0, 0, g.ny, g.nz + 1};
-}
-
 // One thread per particle, face velocities from global memory (the
 // advection alone, and any particle order).
 template <class T, bool FACTORED>
@@ -1141,11 +1165,9 @@ __global__ void __launch_bounds__(256) k_g2p(GridP<T> g, T* __restrict__ pd, lon
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int d[3] = {d0, d1, d2};
-    g2p_particle<T, FACTORED>(g, pd, cap, i, d, do_g2p, do_advect, dt, sp, keys, vals,
-                              [&](const int*, VSrc<T> src[3]) {
-                                  global_sources(g, vx, vy, vz, src);
-                                  return false;
-                              });
+    T q[3] = {pd[i], pd[cap + i], pd[2 * cap + i]};
+    g2p_particle<T, FACTORED, false>(g, pd, cap, i, q, d, do_g2p, do_advect, dt, sp, keys, vals,
+                                     GlobalSrc<T>{{vx, vy, vz}, g.ny, g.nz}, StagedSrc<T>{}, 0);
 }
 
 // G2P + advection over the cell-sorted particles, one CTA per 8^3-cell tile:
@@ -1153,8 +1175,14 @@ __global__ void __launch_bounds__(256) k_g2p(GridP<T> g, T* __restrict__ pd, lon
 // staged once in shared memory with coalesced loads, then every particle of
 // the tile's 64 rows gathers from it.  The gather arithmetic is that of
 // k_g2p (bit-identical in FP32 / FP64, the factored sums in mixed precision).
+// What bounds it: the latency of a particle's chain (position, window, solid
+// distance at the new position) against the warps that fit: ~900 instructions
+// a particle, issue slots half full.  256^3 dam, 24 warps an SM 1.40 ms, 32 (64
+// registers) 1.24, 40 1.25; the unfactored sums spill above 24 (FP64 at 48^3
+// 171, 186, 256 us).  1.85 ms with run-time strides, a serial row count and
+// the id's gather waited for before the velocities'.
 template <class T, bool FACTORED>
-__global__ void __launch_bounds__(256, 3) k_g2p_tile(GridP<T> g, T* __restrict__ pd, long long cap,
+__global__ void __launch_bounds__(256, FACTORED ? 4 : 3) k_g2p_tile(GridP<T> g, T* __restrict__ pd, long long cap,
                                                   const int32_t* __restrict__ cs, int d0, int d1, int d2,
                                                   const T* __restrict__ vx, const T* __restrict__ vy,
                                                   const T* __restrict__ vz, T dt, const T* __restrict__ sp,
@@ -1166,21 +1194,30 @@ __global__ void __launch_bounds__(256, 3) k_g2p_tile(GridP<T> g, T* __restrict__
     __shared__ int rbeg[kTile * kTile];
     const int x0 = blockIdx.z * kTile, y0 = blockIdx.y * kTile, z0 = blockIdx.x * kTile;
     const int zend = min(z0 + kTile, g.nz);
-    if (threadIdx.x < kTile * kTile) {
-        const int rx = x0 + (threadIdx.x >> 3), ry = y0 + (threadIdx.x & 7);
-        int cnt = 0, beg = 0;
-        if (rx < g.nx && ry < g.ny) {
-            const long long c = ((long long)rx * g.ny + ry) * g.nz + z0;
-            beg = cs[c];
-            cnt = cs[c + (zend - z0)] - beg;
+    if (threadIdx.x < 32) {  // the rows' first particles and their running count, two rows a lane
+        int beg[2], cnt[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int r = 2 * threadIdx.x + k, rx = x0 + r / kTile, ry = y0 + r % kTile;
+            beg[k] = cnt[k] = 0;
+            if (rx < g.nx && ry < g.ny) {
+                const long long c = ((long long)rx * g.ny + ry) * g.nz + z0;
+                beg[k] = cs[c];
+                cnt[k] = cs[c + (zend - z0)] - beg[k];
+            }
         }
-        rbeg[threadIdx.x] = beg;
-        roff[threadIdx.x + 1] = cnt;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        roff[0] = 0;
-        for (int r = 0; r < kTile * kTile; ++r) roff[r + 1] += roff[r];
+        int sum = cnt[0] + cnt[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (threadIdx.x >= o) sum += v;
+        }
+        const int r = 2 * threadIdx.x;
+        rbeg[r] = beg[0];
+        rbeg[r + 1] = beg[1];
+        roff[r + 1] = sum - cnt[1];
+        roff[r + 2] = sum;
+        if (threadIdx.x == 0) roff[0] = 0;
     }
     __syncthreads();
     const int total = roff[kTile * kTile];
@@ -1212,20 +1249,13 @@ __global__ void __launch_bounds__(256, 3) k_g2p_tile(GridP<T> g, T* __restrict__
             else hi = mid;
         }
         const long long i = rbeg[lo] + (f - roff[lo]);
-        // the deferred permutation: vals holds it and gets the identity below
-        if (pid_src) pid_dst[i] = pid_src[vals[i]];
-        g2p_particle<T, FACTORED>(g, pd, cap, i, d, 1, 1, dt, sp, keys, vals, [&](const int* ci, VSrc<T> src[3]) {
-            const bool in = ci[0] >= x0 && ci[0] < x0 + kTile && ci[1] >= y0 && ci[1] < y0 + kTile && ci[2] >= z0 &&
-                            ci[2] < zend;
-            if (!in) {  // off the grid: sorted into a clamped cell
-                global_sources(g, vx, vy, vz, src);
-                return false;
-            }
-            src[0] = VSrc<T>{sv, x0 - 1, y0 - 1, z0 - 1, kTile + 2, kTile + 2};
-            src[1] = VSrc<T>{sv + R0, x0 - 1, y0 - 1, z0 - 1, kTile + 3, kTile + 2};
-            src[2] = VSrc<T>{sv + R0 + R1, x0 - 1, y0 - 1, z0 - 1, kTile + 2, kTile + 3};
-            return true;
-        });
+        // the deferred permutation: vals holds it and gets the identity from the advection
+        const int32_t from = pid_src ? vals[i] : 0;
+        T q[3] = {pd[i], pd[cap + i], pd[2 * cap + i]};  // (sorted also while the sort's permutation waits)
+        g2p_particle<T, FACTORED, true>(g, pd, cap, i, q, d, 1, 1, dt, sp, keys, vals,
+                                        GlobalSrc<T>{{vx, vy, vz}, g.ny, g.nz},
+                                        StagedSrc<T>{sv, x0 - 1, y0 - 1, z0 - 1}, zend);
+        if (pid_src) pid_dst[i] = pid_src[from];
     }
 }
 
