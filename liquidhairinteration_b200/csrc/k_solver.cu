@@ -447,7 +447,9 @@ template <class F> __device__ __forceinline__ void for_tiles(const TileK& tk, in
 // for_tiles with a thread's rows of a work unit handed over together:
 // f(x, z, i0, rows, ys) where row k < rows is cell i0 + k * ys * nz (y
 // ascending).  Kernels load every row before using any, so a thread keeps
-// up to 8 rows of loads in flight; per-thread sums keep for_tiles' order.
+// up to 8 rows of loads in flight; per-thread sums keep for_tiles' order.  The
+// kernels' R is the most rows a unit has (kTileY, or 2 on small levels: fewer
+// registers, so more of the launch runs at once).
 template <class F> __device__ __forceinline__ void for_tile_cols(const TileK& tk, int nx, int ny, int nz, F&& f) {
     const int units = *tk.count * tk.ysplit;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -535,8 +537,11 @@ __device__ __forceinline__ void smooth_cell(const LevelK<T>& L, const T* __restr
 // One colour of one level over its active tiles.  A thread owns (x, z) of a
 // tile and the 4 rows y of that colour; a work unit takes every ysplit-th of
 // them.  All loads of a thread's rows are issued before any update.
-template <class T>
-__global__ void __launch_bounds__(kTileThreads, 2) k_sweep(LevelK<T> L, TileK tk, const T* __restrict__ r, T* __restrict__ z,
+// R: rows a thread takes at most.  A small level's units are of one row (R =
+// 1), whose 40 registers let every CTA of the launch run at once; with four
+// rows' registers they came in three waves (93 x 70 x 61: 7.4 -> 5.3 us).
+template <class T, int R>
+__global__ void __launch_bounds__(kTileThreads, R > 1 ? 2 : sizeof(T) == 4 ? 6 : 3) k_sweep(LevelK<T> L, TileK tk, const T* __restrict__ r, T* __restrict__ z,
                                                         T w, int variant, int phase, const int* __restrict__ stop) {
     if (*stop) return;
     const int units = *tk.count * tk.ysplit;
@@ -550,14 +555,14 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_sweep(LevelK<T> L, TileK tk
         if (x >= L.nx || zz >= L.nz) continue;
         const int y0 = ty * kTileY;
         const int yf = y0 + ((phase + x + zz + y0) & 1);
-        Cell7<T, T> c[4];
-        T rv[4];
-        bool act[4];
-        long long idx[4];
+        Cell7<T, T> c[R];
+        T rv[R];
+        bool act[R];
+        long long idx[R];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int y = yf + 2 * k;
-            act[k] = (k % tk.ysplit == sub) && y < L.ny;
+        for (int k = 0; k < R; ++k) {
+            const int row = sub + k * tk.ysplit, y = yf + 2 * row;
+            act[k] = row < 4 && y < L.ny;
             if (act[k]) {
                 idx[k] = ((long long)x * L.ny + y) * L.nz + zz;
                 load7(L, z, idx[k], x, y, zz, c[k]);
@@ -565,7 +570,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_sweep(LevelK<T> L, TileK tk
             }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < R; ++k) {
             T out;
             if (act[k] && smooth7(c[k], rv[k], w, variant, out)) z[idx[k]] = out;
         }
@@ -906,7 +911,7 @@ __global__ void __launch_bounds__(256) k_restrict_dense(LevelK<T> F, const T* __
 
 // CGSolver<3>::Prolong (PressureSolver.cpp:774-794): piecewise-constant,
 // written per fine cell (fine cells beyond 2 * coarse extent get nothing).
-template <class T>
+template <class T, int R>
 __global__ void __launch_bounds__(kTileThreads) k_prolong_t(int fnx, int fny, int fnz, TileK tk, const T* __restrict__ zc,
                                                             int cnx, int cny, int cnz, T* __restrict__ zf,
                                                             const int* __restrict__ stop) {
@@ -914,10 +919,10 @@ __global__ void __launch_bounds__(kTileThreads) k_prolong_t(int fnx, int fny, in
     for_tile_cols(tk, fnx, fny, fnz, [&](int x, int z, long long i0, int yb, int rows, int ys) {
         const long long st = (long long)ys * fnz;
         const int cx = x >> 1, cz = z >> 1;
-        bool on[kTileY];
-        T fv[kTileY], cv[kTileY];
+        bool on[R];
+        T fv[R], cv[R];
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k) {
+        for (int k = 0; k < R; ++k) {
             const int cy = (yb + k * ys) >> 1;
             on[k] = k < rows && cx < cnx && cy < cny && cz < cnz;
             if (on[k]) {
@@ -926,7 +931,7 @@ __global__ void __launch_bounds__(kTileThreads) k_prolong_t(int fnx, int fny, in
             }
         }
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             if (on[k]) zf[i0 + k * st] = fv[k] + cv[k];
     });
 }
@@ -1735,12 +1740,14 @@ __global__ void __launch_bounds__(kTileThreads, 3)
 }
 
 // Ap = A p; p.Ap over the update region; alpha = rz / p.Ap (PressureSolver.cpp:873-888).
-// A thread owns (x, z) of a tile and 8 rows, loaded 4 rows at a time.
-template <class T>
-__global__ void __launch_bounds__(kTileThreads, 2) k_cg_spmv(LevelK<T> L, TileK tk, const T* __restrict__ p, T* __restrict__ ap,
+// A thread owns (x, z) of a tile and 8 rows, loaded 4 rows at a time; on small
+// levels at most R = 2 of them, as in k_sweep (93 x 70 x 61: 13 -> 10 us; both rows in flight at 64 registers: the same).
+template <class T, int R>
+__global__ void __launch_bounds__(kTileThreads, R > 2 ? 2 : sizeof(T) == 4 ? 6 : 3) k_cg_spmv(LevelK<T> L, TileK tk, const T* __restrict__ p, T* __restrict__ ap,
                                                           double* __restrict__ partials, unsigned* __restrict__ counter,
                                                           SolveScalars* __restrict__ sc, CgConf cf) {
     if (sc->stop) return;
+    constexpr int kB = R < 4 ? 1 : 4;
     double v[1] = {0.0};
     const int units = *tk.count * tk.ysplit;
     const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1753,25 +1760,25 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_cg_spmv(LevelK<T> L, TileK 
         if (x >= L.nx || zz >= L.nz) continue;
         const int y0 = ty * kTileY;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            Cell7<T, T> c[4];
-            bool act[4];
-            long long idx[4];
+        for (int h = 0; h < R; h += kB) {
+            Cell7<T, T> c[kB];
+            bool act[kB];
+            long long idx[kB];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int yy = 4 * h + k, y = y0 + yy;
-                act[k] = (yy % tk.ysplit == sub) && y < L.ny;
+            for (int k = 0; k < kB; ++k) {
+                const int yy = sub + (h + k) * tk.ysplit, y = y0 + yy;
+                act[k] = yy < kTileY && y < L.ny;
                 if (act[k]) {
                     idx[k] = ((long long)x * L.ny + y) * L.nz + zz;
                     load7(L, p, idx[k], x, y, zz, c[k]);
                 }
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < kB; ++k) {
                 if (!act[k]) continue;
                 const T a = ax7<T>(c[k]);
                 ap[idx[k]] = a;
-                if (c[k].tc != 0 && in_region(x, y0 + 4 * h + k, zz, L.nx, L.ny, L.nz, cf.region))
+                if (c[k].tc != 0 && in_region(x, y0 + sub + (h + k) * tk.ysplit, zz, L.nx, L.ny, L.nz, cf.region))
                     v[0] += double(c[k].zc) * double(a);
             }
         }
@@ -1784,7 +1791,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_cg_spmv(LevelK<T> L, TileK 
 
 // x += alpha p; r -= alpha Ap; ||r||^2 over the update region; then the
 // stopping rule (PressureSolver.cpp:889-902)
-template <class T, class TX>
+template <class T, class TX, int R>
 __global__ void __launch_bounds__(kTileThreads) k_cg_update_xr(LevelK<T> L, TileK tk, const T* __restrict__ p,
                                                                const T* __restrict__ ap, TX* __restrict__ x,
                                                                T* __restrict__ r, double* __restrict__ partials,
@@ -1798,14 +1805,14 @@ __global__ void __launch_bounds__(kTileThreads) k_cg_update_xr(LevelK<T> L, Tile
     double v[1] = {0.0};
     for_tile_cols(tk, L.nx, L.ny, L.nz, [&](int xi, int zi, long long i0, int yb, int rows, int ys) {
         const long long st = (long long)ys * L.nz;
-        bool on[kTileY];
-        TX xv[kTileY];
-        T pv[kTileY], rv[kTileY], av[kTileY];
+        bool on[R];
+        TX xv[R];
+        T pv[R], rv[R], av[R];
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             on[k] = k < rows && L.type[i0 + k * st] != 0 && in_region(xi, yb + k * ys, zi, L.nx, L.ny, L.nz, cf.region);
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             if (on[k]) {
                 xv[k] = x[i0 + k * st];
                 pv[k] = p[i0 + k * st];
@@ -1813,7 +1820,7 @@ __global__ void __launch_bounds__(kTileThreads) k_cg_update_xr(LevelK<T> L, Tile
                 av[k] = ap[i0 + k * st];
             }
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             if (on[k]) {
                 x[i0 + k * st] = TX(double(xv[k]) + alpha * double(pv[k]));
                 const T rn = T(double(rv[k]) - alpha * double(av[k]));
@@ -1876,7 +1883,7 @@ __global__ void __launch_bounds__(kTileThreads) k_true_residual_final(LevelK<T> 
 // rz_new = r.z over all cells (Array3::Reduce); Ap.z over the update region;
 // beta (PressureSolver.cpp:905-912): Fletcher-Reeves, or Polak-Ribiere
 // -alpha Ap.z / rz_old when flexible
-template <class T>
+template <class T, int R>
 __global__ void __launch_bounds__(kTileThreads) k_cg_dot_rz(LevelK<T> L, TileK tk, const T* __restrict__ r,
                                                             const T* __restrict__ z, const T* __restrict__ ap,
                                                             double* __restrict__ partials, unsigned* __restrict__ counter,
@@ -1885,10 +1892,10 @@ __global__ void __launch_bounds__(kTileThreads) k_cg_dot_rz(LevelK<T> L, TileK t
     double v[2] = {0.0, 0.0};
     for_tile_cols(tk, L.nx, L.ny, L.nz, [&](int xi, int zz, long long i0, int yb, int rows, int ys) {
         const long long st = (long long)ys * L.nz;
-        bool on[kTileY];
-        T zv[kTileY], rv[kTileY], av[kTileY];
+        bool on[R];
+        T zv[R], rv[R], av[R];
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k) {
+        for (int k = 0; k < R; ++k) {
             on[k] = k < rows && L.type[i0 + k * st] != 0 && in_region(xi, yb + k * ys, zz, L.nx, L.ny, L.nz, cf.region);
             if (k < rows) {
                 zv[k] = z[i0 + k * st];
@@ -1896,10 +1903,10 @@ __global__ void __launch_bounds__(kTileThreads) k_cg_dot_rz(LevelK<T> L, TileK t
             }
         }
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             if (on[k]) av[k] = ap[i0 + k * st];
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k) {
+        for (int k = 0; k < R; ++k) {
             if (k >= rows) break;
             v[0] += double(rv[k]) * double(zv[k]);
             if (on[k]) v[1] += double(av[k]) * double(zv[k]);
@@ -1915,25 +1922,25 @@ __global__ void __launch_bounds__(kTileThreads) k_cg_dot_rz(LevelK<T> L, TileK t
 }
 
 // p = z + beta p on fluid cells (PressureSolver.cpp:913-921)
-template <class T>
+template <class T, int R>
 __global__ void __launch_bounds__(kTileThreads) k_cg_update_p(LevelK<T> L, TileK tk, const T* __restrict__ z,
                                                               T* __restrict__ p, const SolveScalars* __restrict__ sc) {
     if (sc->stop) return;
     const double beta = sc->beta;
     for_tile_cols(tk, L.nx, L.ny, L.nz, [&](int x, int zz, long long i0, int yb, int rows, int ys) {
         const long long st = (long long)ys * L.nz;
-        bool on[kTileY];
-        T zv[kTileY], pv[kTileY];
+        bool on[R];
+        T zv[R], pv[R];
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k) on[k] = k < rows && L.type[i0 + k * st] != 0;
+        for (int k = 0; k < R; ++k) on[k] = k < rows && L.type[i0 + k * st] != 0;
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             if (on[k]) {
                 zv[k] = z[i0 + k * st];
                 pv[k] = p[i0 + k * st];
             }
 #pragma unroll
-        for (int k = 0; k < kTileY; ++k)
+        for (int k = 0; k < R; ++k)
             if (on[k]) p[i0 + k * st] = T(double(zv[k]) + beta * double(pv[k]));
     });
 }
@@ -2051,6 +2058,7 @@ static int ysplit_for(int ntiles, int grid, int max_split = kTileY) {
     while (s < max_split && ntiles * s * 2 <= grid) s *= 2;
     return s;
 }
+static bool few_rows(const TileK& tk) { return tk.ysplit >= kTileY / 2; }  // units of at most two rows
 template <class T> static TileK tile_k(const LevelDev<T>& L, const int* count, int grid, int max_split = kTileY) {
     return TileK{L.tiles, count, L.tdim[1], L.tdim[2], ysplit_for(L.ntiles, grid, max_split)};
 }
@@ -2317,7 +2325,8 @@ template <class T, class TX> bool LiquidImpl<T, TX>::smooth(int level, int sweep
     for (int s = 0; s < sweeps; ++s)
         for (int phase = 0; phase < 2; ++phase) {
             auto ps_ = scope(cat);
-            k_sweep<T><<<G, kTileThreads, 0, cur_>>>(lk(L), tk, L.r, L.z, w, sp_.smoother, phase, &sc_->stop);
+            const auto kern = tk.ysplit == 4 ? k_sweep<T, 1> : k_sweep<T, 4>;
+            kern<<<G, kTileThreads, 0, cur_>>>(lk(L), tk, L.r, L.z, w, sp_.smoother, phase, &sc_->stop);
             LHI_LAUNCH_CHECK();
         }
     return false;
@@ -2352,8 +2361,9 @@ template <class T, class TX> void LiquidImpl<T, TX>::prolong_to(int level) {
     const unsigned G = tile_blocks(F, tile_grid_);
     if (C.n == 0 || F.n == 0 || G == 0) return;
     auto ps_ = scope(LHI_KERNEL_PROLONG);
-    k_prolong_t<T><<<G, kTileThreads, 0, cur_>>>(F.nx, F.ny, F.nz, tile_k(F, &sc_->tile_count[level], tile_grid_),
-                                                 C.z, C.nx, C.ny, C.nz, F.z, &sc_->stop);
+    const TileK tk = tile_k(F, &sc_->tile_count[level], tile_grid_);
+    auto kern = few_rows(tk) ? k_prolong_t<T, 2> : k_prolong_t<T, kTileY>;
+    kern<<<G, kTileThreads, 0, cur_>>>(F.nx, F.ny, F.nz, tk, C.z, C.nx, C.ny, C.nz, F.z, &sc_->stop);
     LHI_LAUNCH_CHECK();
 }
 
@@ -2566,14 +2576,16 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_body(unsigned long 
                 tm_sp_[0], tm_sp_[1], tm_sp_[2], tm_sp_[3], tm_sp_[4], tm_sp_[5], L0.nx, L0.ny, L0.nz, L0.tiles,
                 &sc_->tile_count[0], L0.tdim[1], L0.tdim[2], reinterpret_cast<float*>(ap_), partials_, counter_, sc_,
                 cf);
-        else
-            k_cg_spmv<T><<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, partials_, counter_, sc_, cf);
+        else {
+            const auto kern = few_rows(tk) ? k_cg_spmv<T, 2> : k_cg_spmv<T, kTileY>;
+            kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, partials_, counter_, sc_, cf);
+        }
         LHI_LAUNCH_CHECK();
     }
     {
         auto ps_ = scope(LHI_KERNEL_CG_VECTOR);
-        k_cg_update_xr<T, TX><<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, x_, L0.r, partials_, counter_, sc_,
-                                                            cf);
+        const auto kern = few_rows(tk) ? k_cg_update_xr<T, TX, 2> : k_cg_update_xr<T, TX, kTileY>;
+        kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, x_, L0.r, partials_, counter_, sc_, cf);
         LHI_LAUNCH_CHECK();
         if (sp_.true_residual_every > 0) {
             if constexpr (kHiResidual)
@@ -2595,10 +2607,12 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_body(unsigned long 
     {
         auto ps_ = scope(LHI_KERNEL_CG_VECTOR);
         if (!dot_fused_) {
-            k_cg_dot_rz<T><<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, L0.r, L0.z, ap_, partials_, counter_, sc_, cf);
+            const auto kern = few_rows(tk) ? k_cg_dot_rz<T, 2> : k_cg_dot_rz<T, kTileY>;
+            kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, L0.r, L0.z, ap_, partials_, counter_, sc_, cf);
             LHI_LAUNCH_CHECK();
         }
-        k_cg_update_p<T><<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, L0.z, p_, sc_);
+        const auto kern = few_rows(tk) ? k_cg_update_p<T, 2> : k_cg_update_p<T, kTileY>;
+        kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, L0.z, p_, sc_);
         LHI_LAUNCH_CHECK();
     }
 }
@@ -2847,8 +2861,10 @@ template <class T, class TX> double LiquidImpl<T, TX>::spmv_p(int* tma) {
                 tm_sp_[0], tm_sp_[1], tm_sp_[2], tm_sp_[3], tm_sp_[4], tm_sp_[5], L0.nx, L0.ny, L0.nz, L0.tiles,
                 &sc_->tile_count[0], L0.tdim[1], L0.tdim[2], reinterpret_cast<float*>(ap_), partials_, counter_, sc_,
                 cf);
-        else
-            k_cg_spmv<T><<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, partials_, counter_, sc_, cf);
+        else {
+            const auto kern = few_rows(tk) ? k_cg_spmv<T, 2> : k_cg_spmv<T, kTileY>;
+            kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, partials_, counter_, sc_, cf);
+        }
         LHI_LAUNCH_CHECK();
     }
     read_scalars();
