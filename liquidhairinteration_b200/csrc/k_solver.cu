@@ -534,46 +534,33 @@ __device__ __forceinline__ void smooth_cell(const LevelK<T>& L, const T* __restr
     else z[i] = T((1.0 - double(w)) * double(z[i]) + double(T(w * term)));
 }
 
-// One colour of one level over its active tiles.  A thread owns (x, z) of a
-// tile and the 4 rows y of that colour; a work unit takes every ysplit-th of
-// them.  All loads of a thread's rows are issued before any update.
-// R: rows a thread takes at most.  A small level's units are of one row (R =
-// 1), whose 40 registers let every CTA of the launch run at once; with four
-// rows' registers they came in three waves (93 x 70 x 61: 7.4 -> 5.3 us).
-template <class T, int R>
-__global__ void __launch_bounds__(kTileThreads, R > 1 ? 2 : sizeof(T) == 4 ? 6 : 3) k_sweep(LevelK<T> L, TileK tk, const T* __restrict__ r, T* __restrict__ z,
-                                                        T w, int variant, int phase, const int* __restrict__ stop) {
+// One colour of one level over its active tiles.  A work unit is one of the
+// four rows y of that colour in a tile, a thread its cell at (x, z).  Latency
+// bounds it: one row a thread takes 40 registers, so that six CTAs an SM are
+// at work (FP64: three); four rows, loaded ahead, took 128 and two CTAs
+// (93 x 70 x 61: 7.4 -> 5.3 us; a PCG iteration of 125 x 141 x 99 187 -> 167,
+// of 128^3 in FP64 236 -> 213).
+constexpr int kSweepSplit = kTileY / 2;
+template <class T>
+__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? 6 : 3)
+    k_sweep(LevelK<T> L, TileK tk, const T* __restrict__ r, T* __restrict__ z, T w, int variant, int phase,
+            const int* __restrict__ stop) {
     if (*stop) return;
-    const int units = *tk.count * tk.ysplit;
+    const int units = *tk.count * kSweepSplit;
     const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
-        const int t = u / tk.ysplit, sub = u - t * tk.ysplit;
+        const int t = u / kSweepSplit, row = u - t * kSweepSplit;
         const int id = tk.ids[t];
         const int tz = id % tk.tdz, rest = id / tk.tdz;
         const int ty = rest % tk.tdy, tx = rest / tk.tdy;
         const int x = tx * kTileX + wp, zz = tz * kTileZ + lane;
-        if (x >= L.nx || zz >= L.nz) continue;
-        const int y0 = ty * kTileY;
-        const int yf = y0 + ((phase + x + zz + y0) & 1);
-        Cell7<T, T> c[R];
-        T rv[R];
-        bool act[R];
-        long long idx[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const int row = sub + k * tk.ysplit, y = yf + 2 * row;
-            act[k] = row < 4 && y < L.ny;
-            if (act[k]) {
-                idx[k] = ((long long)x * L.ny + y) * L.nz + zz;
-                load7(L, z, idx[k], x, y, zz, c[k]);
-                rv[k] = r[idx[k]];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            T out;
-            if (act[k] && smooth7(c[k], rv[k], w, variant, out)) z[idx[k]] = out;
-        }
+        const int y0 = ty * kTileY, y = y0 + ((phase + x + zz + y0) & 1) + 2 * row;
+        if (x >= L.nx || zz >= L.nz || y >= L.ny) continue;
+        const long long i = ((long long)x * L.ny + y) * L.nz + zz;
+        Cell7<T, T> c;
+        load7(L, z, i, x, y, zz, c);
+        T out;
+        if (smooth7(c, r[i], w, variant, out)) z[i] = out;
     }
 }
 
@@ -1740,49 +1727,21 @@ __global__ void __launch_bounds__(kTileThreads, 3)
 }
 
 // Ap = A p; p.Ap over the update region; alpha = rz / p.Ap (PressureSolver.cpp:873-888).
-// A thread owns (x, z) of a tile and 8 rows, loaded 4 rows at a time; on small
-// levels at most R = 2 of them, as in k_sweep (93 x 70 x 61: 13 -> 10 us; both rows in flight at 64 registers: the same).
-template <class T, int R>
-__global__ void __launch_bounds__(kTileThreads, R > 2 ? 2 : sizeof(T) == 4 ? 6 : 3) k_cg_spmv(LevelK<T> L, TileK tk, const T* __restrict__ p, T* __restrict__ ap,
-                                                          double* __restrict__ partials, unsigned* __restrict__ counter,
-                                                          SolveScalars* __restrict__ sc, CgConf cf) {
+// A work unit is every ysplit-th row (four or eight) of a tile, row by row, for
+// the reason of k_sweep (93 x 70 x 61: 13 us with four rows loaded ahead, 10 now).
+template <class T>
+__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? 6 : 3)
+    k_cg_spmv(LevelK<T> L, TileK tk, const T* __restrict__ p, T* __restrict__ ap, double* __restrict__ partials,
+              unsigned* __restrict__ counter, SolveScalars* __restrict__ sc, CgConf cf) {
     if (sc->stop) return;
-    constexpr int kB = R < 4 ? 1 : 4;
     double v[1] = {0.0};
-    const int units = *tk.count * tk.ysplit;
-    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-        const int t = u / tk.ysplit, sub = u - t * tk.ysplit;
-        const int id = tk.ids[t];
-        const int tz = id % tk.tdz, rest = id / tk.tdz;
-        const int ty = rest % tk.tdy, tx = rest / tk.tdy;
-        const int x = tx * kTileX + wp, zz = tz * kTileZ + lane;
-        if (x >= L.nx || zz >= L.nz) continue;
-        const int y0 = ty * kTileY;
-#pragma unroll
-        for (int h = 0; h < R; h += kB) {
-            Cell7<T, T> c[kB];
-            bool act[kB];
-            long long idx[kB];
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                const int yy = sub + (h + k) * tk.ysplit, y = y0 + yy;
-                act[k] = yy < kTileY && y < L.ny;
-                if (act[k]) {
-                    idx[k] = ((long long)x * L.ny + y) * L.nz + zz;
-                    load7(L, p, idx[k], x, y, zz, c[k]);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                if (!act[k]) continue;
-                const T a = ax7<T>(c[k]);
-                ap[idx[k]] = a;
-                if (c[k].tc != 0 && in_region(x, y0 + sub + (h + k) * tk.ysplit, zz, L.nx, L.ny, L.nz, cf.region))
-                    v[0] += double(c[k].zc) * double(a);
-            }
-        }
-    }
+    for_tiles(tk, L.nx, L.ny, L.nz, [&](int x, int y, int z, long long i) {
+        Cell7<T, T> c;
+        load7(L, p, i, x, y, z, c);
+        const T a = ax7<T>(c);
+        ap[i] = a;
+        if (c.tc != 0 && in_region(x, y, z, L.nx, L.ny, L.nz, cf.region)) v[0] += double(c.zc) * double(a);
+    });
     double tot[1];
     if (!grid_sum_last<1>(v, partials, counter, tot)) return;
     sc->denom = tot[0];
@@ -2051,22 +2010,29 @@ __global__ void k_loss_grad(LevelK<T> L, const float* __restrict__ e, int batch,
 }  // namespace
 
 // ------------------------------------------------------------- host side
-// Work units per tile: enough units to fill `grid` CTAs, at most max_split
-// (4 for the colour sweeps, whose threads own 4 rows; 8 otherwise).
-static int ysplit_for(int ntiles, int grid, int max_split = kTileY) {
-    int s = 1;
-    while (s < max_split && ntiles * s * 2 <= grid) s *= 2;
+// Work units per tile: enough units to fill `grid` CTAs, at least min_split.
+static int ysplit_for(int ntiles, int grid, int min_split) {
+    int s = min_split;
+    while (s < kTileY && ntiles * s * 2 <= grid) s *= 2;
     return s;
 }
-static bool few_rows(const TileK& tk) { return tk.ysplit >= kTileY / 2; }  // units of at most two rows
-template <class T> static TileK tile_k(const LevelDev<T>& L, const int* count, int grid, int max_split = kTileY) {
-    return TileK{L.tiles, count, L.tdim[1], L.tdim[2], ysplit_for(L.ntiles, grid, max_split)};
+template <class T> static TileK tile_k(const LevelDev<T>& L, const int* count, int grid, int min_split = 1) {
+    return TileK{L.tiles, count, L.tdim[1], L.tdim[2], ysplit_for(L.ntiles, grid, min_split)};
 }
 // persistent CTAs for a tile kernel on level L (0 when the level is empty)
-template <class T> static unsigned tile_blocks(const LevelDev<T>& L, int grid, int max_split = kTileY) {
-    const long long units = (long long)L.ntiles * ysplit_for(L.ntiles, grid, max_split);
+template <class T> static unsigned tile_blocks(const LevelDev<T>& L, int grid, int min_split = 1) {
+    const long long units = (long long)L.ntiles * ysplit_for(L.ntiles, grid, min_split);
     return unsigned(std::min<long long>(units, grid));
 }
+constexpr int kFewRows = 2;              // rows of a unit at a split of kSplit
+constexpr int kSplit = kTileY / kFewRows;  // of k_cg_spmv and, on levels of few tiles, of the column kernels
+// The column kernels (prolongation, CG vectors) hold all rows of a unit: two on
+// levels of up to kColsTiles tiles, where more CTAs at work count for more than
+// the loads a thread has in flight, eight above.  A PCG iteration with two and
+// with eight: 432 tiles (96^3, FP64) 163 and 169 us, 1024 (128^3, FP64) 213 and
+// 218, 1152 (125 x 141 x 99) 161.0 and 159.3, 2000 (160^3, mixed) 231 and 229.5.
+constexpr int kColsTiles = 1024;
+template <class T> static int cols_split(const LevelDev<T>& L) { return L.ntiles <= kColsTiles ? kSplit : 1; }
 
 template <class T, class TX> double LiquidImpl<T, TX>::read_scalar(const double* dptr) {
     double v;
@@ -2300,7 +2266,7 @@ template <class T, class TX> void LiquidImpl<T, TX>::build_tiles() {
 
 template <class T, class TX> bool LiquidImpl<T, TX>::smooth(int level, int sweeps, bool final_dot) {
     LevelDev<T>& L = lv_[level];
-    const unsigned G = tile_blocks(L, tile_grid_, 4);
+    const unsigned G = unsigned(std::min((long long)L.ntiles * kSweepSplit, (long long)tile_grid_));
     if (L.n == 0 || sweeps <= 0 || G == 0) return false;
     const T w = T(sp_.smoothing_factor);
     const int cat = (level == 0) ? LHI_KERNEL_SMOOTH_FINE : LHI_KERNEL_SMOOTH_COARSE;
@@ -2321,12 +2287,11 @@ template <class T, class TX> bool LiquidImpl<T, TX>::smooth(int level, int sweep
         }
         return final_dot;
     }
-    const TileK tk = tile_k(L, &sc_->tile_count[level], tile_grid_, 4);
+    const TileK tk = tile_k(L, &sc_->tile_count[level], tile_grid_);
     for (int s = 0; s < sweeps; ++s)
         for (int phase = 0; phase < 2; ++phase) {
             auto ps_ = scope(cat);
-            const auto kern = tk.ysplit == 4 ? k_sweep<T, 1> : k_sweep<T, 4>;
-            kern<<<G, kTileThreads, 0, cur_>>>(lk(L), tk, L.r, L.z, w, sp_.smoother, phase, &sc_->stop);
+            k_sweep<T><<<G, kTileThreads, 0, cur_>>>(lk(L), tk, L.r, L.z, w, sp_.smoother, phase, &sc_->stop);
             LHI_LAUNCH_CHECK();
         }
     return false;
@@ -2358,11 +2323,11 @@ template <class T, class TX> void LiquidImpl<T, TX>::restrict_to(int level) {
 template <class T, class TX> void LiquidImpl<T, TX>::prolong_to(int level) {
     LevelDev<T>& C = lv_[level + 1];
     LevelDev<T>& F = lv_[level];
-    const unsigned G = tile_blocks(F, tile_grid_);
+    const unsigned G = tile_blocks(F, tile_grid_, cols_split(F));
     if (C.n == 0 || F.n == 0 || G == 0) return;
     auto ps_ = scope(LHI_KERNEL_PROLONG);
-    const TileK tk = tile_k(F, &sc_->tile_count[level], tile_grid_);
-    auto kern = few_rows(tk) ? k_prolong_t<T, 2> : k_prolong_t<T, kTileY>;
+    const TileK tk = tile_k(F, &sc_->tile_count[level], tile_grid_, cols_split(F));
+    const auto kern = tk.ysplit >= kSplit ? k_prolong_t<T, kFewRows> : k_prolong_t<T, kTileY>;
     kern<<<G, kTileThreads, 0, cur_>>>(F.nx, F.ny, F.nz, tk, C.z, C.nx, C.ny, C.nz, F.z, &sc_->stop);
     LHI_LAUNCH_CHECK();
 }
@@ -2566,8 +2531,8 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_init(unsigned long 
 // One PCG iteration (PressureSolver.cpp:870-922).
 template <class T, class TX> void LiquidImpl<T, TX>::enqueue_body(unsigned long long cond, int use_cond) {
     LevelDev<T>& L0 = lv_[0];
-    const TileK tk = tile_k(L0, &sc_->tile_count[0], tile_grid_);
-    const unsigned G = std::max(1u, tile_blocks(L0, tile_grid_));
+    const TileK tk = tile_k(L0, &sc_->tile_count[0], tile_grid_, cols_split(L0));
+    const unsigned G = std::max(1u, tile_blocks(L0, tile_grid_, cols_split(L0)));
     const CgConf cf = make_conf(sp_, cond, use_cond);
     {
         auto ps_ = scope(LHI_KERNEL_SPMV);
@@ -2576,15 +2541,14 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_body(unsigned long 
                 tm_sp_[0], tm_sp_[1], tm_sp_[2], tm_sp_[3], tm_sp_[4], tm_sp_[5], L0.nx, L0.ny, L0.nz, L0.tiles,
                 &sc_->tile_count[0], L0.tdim[1], L0.tdim[2], reinterpret_cast<float*>(ap_), partials_, counter_, sc_,
                 cf);
-        else {
-            const auto kern = few_rows(tk) ? k_cg_spmv<T, 2> : k_cg_spmv<T, kTileY>;
-            kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, partials_, counter_, sc_, cf);
-        }
+        else
+            k_cg_spmv<T><<<std::max(1u, tile_blocks(L0, tile_grid_, kSplit)), kTileThreads, 0, cur_>>>(
+                lk(L0), tile_k(L0, &sc_->tile_count[0], tile_grid_, kSplit), p_, ap_, partials_, counter_, sc_, cf);
         LHI_LAUNCH_CHECK();
     }
     {
         auto ps_ = scope(LHI_KERNEL_CG_VECTOR);
-        const auto kern = few_rows(tk) ? k_cg_update_xr<T, TX, 2> : k_cg_update_xr<T, TX, kTileY>;
+        const auto kern = tk.ysplit >= kSplit ? k_cg_update_xr<T, TX, kFewRows> : k_cg_update_xr<T, TX, kTileY>;
         kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, x_, L0.r, partials_, counter_, sc_, cf);
         LHI_LAUNCH_CHECK();
         if (sp_.true_residual_every > 0) {
@@ -2607,11 +2571,11 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_body(unsigned long 
     {
         auto ps_ = scope(LHI_KERNEL_CG_VECTOR);
         if (!dot_fused_) {
-            const auto kern = few_rows(tk) ? k_cg_dot_rz<T, 2> : k_cg_dot_rz<T, kTileY>;
+            const auto kern = tk.ysplit >= kSplit ? k_cg_dot_rz<T, kFewRows> : k_cg_dot_rz<T, kTileY>;
             kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, L0.r, L0.z, ap_, partials_, counter_, sc_, cf);
             LHI_LAUNCH_CHECK();
         }
-        const auto kern = few_rows(tk) ? k_cg_update_p<T, 2> : k_cg_update_p<T, kTileY>;
+        const auto kern = tk.ysplit >= kSplit ? k_cg_update_p<T, kFewRows> : k_cg_update_p<T, kTileY>;
         kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, L0.z, p_, sc_);
         LHI_LAUNCH_CHECK();
     }
@@ -2861,10 +2825,9 @@ template <class T, class TX> double LiquidImpl<T, TX>::spmv_p(int* tma) {
                 tm_sp_[0], tm_sp_[1], tm_sp_[2], tm_sp_[3], tm_sp_[4], tm_sp_[5], L0.nx, L0.ny, L0.nz, L0.tiles,
                 &sc_->tile_count[0], L0.tdim[1], L0.tdim[2], reinterpret_cast<float*>(ap_), partials_, counter_, sc_,
                 cf);
-        else {
-            const auto kern = few_rows(tk) ? k_cg_spmv<T, 2> : k_cg_spmv<T, kTileY>;
-            kern<<<G, kTileThreads, 0, cur_>>>(lk(L0), tk, p_, ap_, partials_, counter_, sc_, cf);
-        }
+        else
+            k_cg_spmv<T><<<std::max(1u, tile_blocks(L0, tile_grid_, kSplit)), kTileThreads, 0, cur_>>>(
+                lk(L0), tile_k(L0, &sc_->tile_count[0], tile_grid_, kSplit), p_, ap_, partials_, counter_, sc_, cf);
         LHI_LAUNCH_CHECK();
     }
     read_scalars();
