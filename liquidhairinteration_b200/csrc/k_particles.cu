@@ -583,7 +583,7 @@ __device__ __forceinline__ void p2g_add(double2* p, int stride, const double (&w
 // regrouped and fused and particles are summed in another order, so P2G
 // matches the reference to rounding, not bit for bit.  No per-particle
 // global atomics.
-// What bounds it: shared-memory wavefronts (23 a particle, 75% of the pipe's
+// What bounds it: shared-memory wavefronts (23 a particle, 92% of the pipe's
 // rate: a walking lane receives 48 bytes for its 4 nodes, 12 wavefronts a
 // warp whatever the lanes share), then issue (55 instructions a particle).
 // 256^3 dam break, 32.2 M particles: 2.87 ms; 3.08 ms with separate
