@@ -1267,7 +1267,6 @@ static void free_buffers(NetBuffers& b) {
 
 LearnedNet::~LearnedNet() {
     free_buffers(b_);
-    free_plan();
     auto F = [](void* p) {
         if (p) cudaFree(p);
     };
@@ -1477,28 +1476,6 @@ void launch_wgrad(const uint16_t* g, int cout, int cout_real, const uint16_t* in
 }
 }  // namespace
 
-static long long brick_tiles(const int d[3]) { return (long long)d[0] * ((d[1] + 15) / 16) * ((d[2] + 7) / 8); }
-
-void LearnedNet::free_plan() {
-    for (auto& p : mask_) {
-        if (p) cudaFree(p);
-        p = nullptr;
-    }
-    for (auto& p : tflag_) {
-        if (p) cudaFree(p);
-        p = nullptr;
-    }
-    for (auto& p : tlist_) {
-        if (p) cudaFree(p);
-        p = nullptr;
-    }
-    if (tcount_) cudaFree(tcount_);
-    tcount_ = nullptr;
-    plan_type_ = nullptr;
-    plan_cap_vox0_ = 0;
-    for (int& d : plan_dims_) d = 0;
-}
-
 // Needed voxel sets, from the output back to the input (F = type != 0;
 // dil = one-voxel dilation; up = coarse voxels with a needed child;
 // down = fine voxels with a needed parent):
@@ -1518,21 +1495,14 @@ void LearnedNet::plan_sparse(const int dims[3], const uint8_t* type, cudaStream_
     const int* d0 = b_.dims[0];
     const int* d1 = b_.dims[1];
     const int* d2 = b_.dims[2];
-    const long long V0 = b_.vox[0], V1 = b_.vox[1], V2 = b_.vox[2];
-    if (plan_cap_vox0_ != V0) {
-        free_plan();
-        const long long vl[7] = {V0, V0, V1, V1, V2, V2, V0};
-        for (int i = 0; i < 7; ++i) LHI_CUDA(cudaMalloc(&mask_[i], size_t(std::max(1LL, vl[i]))));
-        const int* dl[3] = {d0, d1, d2};
-        for (int l = 0; l < 3; ++l) LHI_CUDA(cudaMalloc(&tflag_[l], size_t(std::max(1LL, brick_tiles(dl[l])))));
-        // list levels: the six convolutions' outputs, then the input
-        // channels (0), pool to 1, pool to 2, upsample to 1, upsample to 0
-        const int lvl[kPlanLists] = {0, 1, 2, 1, 0, 0, 0, 1, 2, 1, 0};
-        for (int l = 0; l < kPlanLists; ++l)
-            LHI_CUDA(cudaMalloc(&tlist_[l], sizeof(int32_t) * size_t(std::max(1LL, brick_tiles(dl[lvl[l]])))));
-        LHI_CUDA(cudaMalloc(&tcount_, sizeof(int) * kPlanLists));
-        plan_cap_vox0_ = V0;
-    }
+    const long long V0 = b_.vox[0];
+    plan_type_ = nullptr;  // no plan until this one is complete
+    plan_mem_.fit(plan_bytes(net_levels(dims)));
+    size_t m = 0;
+    for (auto& p : mask_) p = plan_mem_.at<uint8_t>(m++);
+    for (auto& p : tflag_) p = plan_mem_.at<uint8_t>(m++);
+    for (auto& p : tlist_) p = plan_mem_.at<int32_t>(m++);
+    tcount_ = plan_mem_.at<int>(m);
     uint8_t *A = mask_[0], *B = mask_[1], *P = mask_[2], *Q = mask_[3], *U = mask_[4], *W = mask_[5];
     uint8_t* S = mask_[6];  // the dilations' intermediate (sized for level 0, used at every level)
     LHI_CUDA(cudaMemsetAsync(tcount_, 0, sizeof(int) * kPlanLists, s));
@@ -1609,8 +1579,8 @@ void LearnedNet::plan_sparse(const int dims[3], const uint8_t* type, cudaStream_
 void LearnedNet::forward(const int dims[3], const float* r, const uint8_t* type, const uint8_t* solid, float* z,
                          double scale_fixed, cudaStream_t s, bool sparse) {
     ensure(dims);
-    sparse = sparse && sparse_enabled_ && plan_type_ == type && plan_cap_vox0_ == b_.vox[0] &&
-             plan_dims_[0] == dims[0] && plan_dims_[1] == dims[1] && plan_dims_[2] == dims[2];
+    sparse = sparse && sparse_enabled_ && plan_type_ == type && plan_dims_[0] == dims[0] &&
+             plan_dims_[1] == dims[1] && plan_dims_[2] == dims[2];
     auto TL = [&](int l) -> const int32_t* { return sparse ? tlist_[l] : nullptr; };
     auto TC = [&](int l) -> const int* { return sparse ? tcount_ + l : nullptr; };
     if (wfmt_stale_) format_weights(s);

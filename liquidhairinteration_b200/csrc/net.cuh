@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "net_buffers.h"
 
 namespace lhi {
 
@@ -75,6 +76,16 @@ __host__ __device__ __forceinline__ float bf16_float(uint16_t b) {
 struct NetStatus {
     int timeout;  // a bounded wait on the tensor-core pipeline gave up
     int pad[7];
+};
+
+// The device's memory for a BufferSet.
+struct DeviceMem {
+    static void* take(size_t n) {
+        void* p = nullptr;
+        LHI_CUDA(cudaMalloc(&p, n));
+        return p;
+    }
+    static void give(void* p) { cudaFree(p); }
 };
 
 // Device buffers of one network applied at one grid size (level dims n0,
@@ -154,16 +165,16 @@ public:
     // stage (kPlanInput .. kPlanUp0: the input channels, the two poolings,
     // the two upsamplings)
     static constexpr int kPlanInput = kNetLayers, kPlanPool0 = kNetLayers + 1, kPlanPool1 = kNetLayers + 2,
-                         kPlanUp1 = kNetLayers + 3, kPlanUp0 = kNetLayers + 4, kPlanLists = kNetLayers + 5;
+                         kPlanUp1 = kNetLayers + 3, kPlanUp0 = kNetLayers + 4;
+    static_assert(kPlanUp0 + 1 == kPlanLists, "a list per layer and elementwise stage");
     bool sparse_enabled_ = true;
     const uint8_t* plan_type_ = nullptr;
     int plan_dims_[3] = {0, 0, 0};
-    uint8_t* mask_[7] = {};
-    uint8_t* tflag_[3] = {};
+    BufferSet<DeviceMem> plan_mem_;  // what the next four point into
+    uint8_t* mask_[kPlanMasks] = {};
+    uint8_t* tflag_[kPlanFlags] = {};
     int32_t* tlist_[kPlanLists] = {};
     int* tcount_ = nullptr;  // [kPlanLists] on the device
-    long long plan_cap_vox0_ = 0;
-    void free_plan();
 };
 
 // Limit of the brick convolution's pipeline waits on the current device.
