@@ -1256,17 +1256,7 @@ LearnedNet::LearnedNet(uint64_t seed) {
     LHI_CUDA(cudaFuncSetAttribute(k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
 }
 
-static void free_buffers(NetBuffers& b) {
-    auto F = [](void* p) {
-        if (p) cudaFree(p);
-    };
-    F(b.a0), F(b.h0), F(b.p0), F(b.h1), F(b.p1), F(b.h2), F(b.q1), F(b.u1), F(b.q0), F(b.u0), F(b.y), F(b.dx), F(b.acc);
-    for (int l = 0; l < kNetLayers; ++l) F(b.g[l]);
-    b = NetBuffers();
-}
-
 LearnedNet::~LearnedNet() {
-    free_buffers(b_);
     auto F = [](void* p) {
         if (p) cudaFree(p);
     };
@@ -1307,43 +1297,25 @@ void set_net_wait_limit_ns(unsigned long long ns) {
 }
 
 void LearnedNet::ensure(const int dims[3]) {
-    int d1[3], d2[3];
-    for (int a = 0; a < 3; ++a) {
-        d1[a] = dims[a] / 2;
-        d2[a] = d1[a] / 2;
+    for (int a = 0; a < 3; ++a)
         if (dims[a] < 4) throw std::invalid_argument("learned preconditioner: grid below 4 cells on an axis");
+    if (layer_mem_.fits(dims)) return;
+    const NetLevels n = net_levels(dims);
+    b_ = NetBuffers();  // no grid's, until every buffer is there
+    layer_mem_.fit(dims, layer_bytes(n));
+    NetBuffers b;
+    size_t m = 0;
+    for (uint16_t** p : {&b.a0, &b.h0, &b.p0, &b.h1, &b.p1, &b.h2, &b.q1, &b.u1, &b.q0, &b.u0})
+        *p = layer_mem_.at<uint16_t>(m++);
+    b.y = layer_mem_.at<float>(m++);
+    for (uint16_t*& p : b.g) p = layer_mem_.at<uint16_t>(m++);
+    b.dx = layer_mem_.at<float>(m++);
+    b.acc = layer_mem_.at<float>(m);
+    for (int l = 0; l < 3; ++l) {
+        for (int a = 0; a < 3; ++a) b.dims[l][a] = n.d[l][a];
+        b.vox[l] = n.vox(l);
     }
-    const long long v0 = (long long)dims[0] * dims[1] * dims[2];
-    bool same = true;
-    for (int a = 0; a < 3; ++a) same = same && b_.dims[0][a] == dims[a];
-    if (same && b_.cap_vox0 == v0) return;
-    free_buffers(b_);
-    for (int a = 0; a < 3; ++a) {
-        b_.dims[0][a] = dims[a];
-        b_.dims[1][a] = d1[a];
-        b_.dims[2][a] = d2[a];
-    }
-    b_.vox[0] = v0;
-    b_.vox[1] = (long long)d1[0] * d1[1] * d1[2];
-    b_.vox[2] = (long long)d2[0] * d2[1] * d2[2];
-    b_.cap_vox0 = v0;
-    const long long V0 = b_.vox[0], V1 = std::max(1LL, b_.vox[1]), V2 = std::max(1LL, b_.vox[2]);
-    auto A16 = [](uint16_t** p, long long n) { LHI_CUDA(cudaMalloc(p, sizeof(uint16_t) * size_t(n))); };
-    A16(&b_.a0, V0 * 16);
-    A16(&b_.h0, V0 * 16);
-    A16(&b_.p0, V1 * 16);
-    A16(&b_.h1, V1 * 32);
-    A16(&b_.p1, V2 * 32);
-    A16(&b_.h2, V2 * 64);
-    A16(&b_.q1, V1 * 64);
-    A16(&b_.u1, V1 * 32);
-    A16(&b_.q0, V0 * 32);
-    A16(&b_.u0, V0 * 16);
-    LHI_CUDA(cudaMalloc(&b_.y, sizeof(float) * V0));
-    const long long gsz[kNetLayers] = {V0 * 16, V1 * 32, V2 * 64, V1 * 32, V0 * 16, V0 * 16};
-    for (int l = 0; l < kNetLayers; ++l) A16(&b_.g[l], gsz[l]);
-    LHI_CUDA(cudaMalloc(&b_.dx, sizeof(float) * std::max(V0 * 32, V1 * 64)));
-    LHI_CUDA(cudaMalloc(&b_.acc, sizeof(float) * std::max(V1 * 32, V2 * 64)));
+    b_ = b;
 }
 
 void LearnedNet::format_weights(cudaStream_t s) {

@@ -93,7 +93,6 @@ struct DeviceMem {
 struct NetBuffers {
     int dims[3][3] = {};
     long long vox[3] = {0, 0, 0};
-    long long cap_vox0 = 0;  // allocation size (voxels of level 0)
     // activations (BF16 channels-last)
     uint16_t* a0 = nullptr;  // 16 ch, L0
     uint16_t* h0 = nullptr;  // 16, L0
@@ -148,6 +147,7 @@ public:
     long long wbwd_off_[kNetLayers] = {};
     bool wfmt_stale_ = true;
     bool relu_ = false;         // activation between layers: ReLU, or none (a linear network)
+    GridBuffers<DeviceMem> layer_mem_;  // what b_ points into
     NetBuffers b_;
     const uint8_t* last_type_ = nullptr;  // cell types of the last forward (device)
     NetStatus* status_ = nullptr;

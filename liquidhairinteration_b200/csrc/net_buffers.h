@@ -1,6 +1,6 @@
 // net_buffers.h -- device buffers that are taken and given back together, and
-// the sizes of those a network's sparse plan needs.  Host arithmetic only:
-// tests/cpp/net_buffers_check.cpp runs it without a GPU.
+// the sizes of those a network's layers and its sparse plan need.  Host
+// arithmetic only: tests/cpp/net_buffers_check.cpp runs it without a GPU.
 #pragma once
 
 #include <algorithm>
@@ -54,6 +54,25 @@ private:
     std::vector<size_t> cap_;
 };
 
+// A set laid out for one grid: another grid gives it back and takes its own,
+// and it is no grid's after a failed allocation.
+template <class Mem> class GridBuffers {
+public:
+    bool fits(const int dims[3]) const { return dims[0] == dims_[0] && dims[1] == dims_[1] && dims[2] == dims_[2]; }
+    void fit(const int dims[3], const std::vector<size_t>& bytes) {
+        for (int& d : dims_) d = 0;
+        set_.release();
+        set_.fit(bytes);
+        for (int a = 0; a < 3; ++a) dims_[a] = dims[a];
+    }
+    template <class T> T* at(size_t i) const { return set_.template at<T>(i); }
+    const BufferSet<Mem>& set() const { return set_; }
+
+private:
+    BufferSet<Mem> set_;
+    int dims_[3] = {0, 0, 0};
+};
+
 // A grid's three levels of the network: every axis halved, rounded down.
 struct NetLevels {
     int d[3][3];
@@ -67,6 +86,16 @@ inline NetLevels net_levels(const int dims[3]) {
         n.d[2][a] = n.d[1][a] / 2;
     }
     return n;
+}
+
+// The layers' buffers, in NetBuffers' order: BF16 activations a0 .. u0, FP32 y,
+// BF16 gradients g[0 .. 5], FP32 dx and acc.
+inline std::vector<size_t> layer_bytes(const NetLevels& n) {
+    const size_t V0 = size_t(n.vox(0)), V1 = size_t(n.vox(1)), V2 = size_t(n.vox(2));
+    return {V0 * 32,  V0 * 32, V1 * 32, V1 * 64, V2 * 64,  V2 * 128,  // a0 h0 p0 h1 p1 h2
+            V1 * 128, V1 * 64, V0 * 64, V0 * 32, V0 * 4,              // q1 u1 q0 u0 y
+            V0 * 32,  V1 * 64, V2 * 128, V1 * 64, V0 * 32, V0 * 32,   // g
+            std::max(V0 * 128, V1 * 256), std::max(V1 * 128, V2 * 256)};
 }
 
 // Brick tiles of a level: one x plane, 16 y, 8 z.  Grids of equal volume can

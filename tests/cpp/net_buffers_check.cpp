@@ -3,7 +3,8 @@
 // of its sparse plan, at least what the plan's kernels write for the new grid
 // (counted here from the kernels' own indices, voxel by voxel), also where
 // the grids have equal volume; a set of buffers is whole or empty after a
-// failed allocation.  Built and run by tests/test_cpu_net_buffers.py.
+// failed allocation, and a network's layers are then no grid's, so that the
+// next call takes them again instead of using what is missing.  Built and run by tests/test_cpu_net_buffers.py.
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -96,6 +97,31 @@ int main() {
         check(threw && s.size() == 0 && Mem::live.empty(), "held after a failed allocation", k, 0, 0);
         s.fit(plan_bytes(net_levels(large)));
         check_plan(s, large);
+    }
+    // the same of a network's layers: 19 buffers
+    for (int k = 0; k < 19; ++k) {
+        GridBuffers<Mem> g;
+        const int small[3] = {4, 4, 4}, large[3] = {16, 17, 16};
+        auto fit = [&](const int* d) { g.fit(d, layer_bytes(net_levels(d))); };
+        check(!g.fits(small), "layers of no grid", k, 0, 0);
+        fit(small);
+        check(g.fits(small) && !g.fits(large), "layers of the grid", k, 0, 0);
+        for (int again = 0; again < 2; ++again) {  // refused each time, not taken for laid out
+            Mem::fail_at = Mem::takes + k;
+            bool threw = false;
+            try {
+                fit(large);
+            } catch (const std::bad_alloc&) {
+                threw = true;
+            }
+            Mem::fail_at = -1;
+            check(threw && Mem::live.empty() && !g.fits(small) && !g.fits(large), "layers held after a failed allocation", k,
+                  again, 0);
+        }
+        fit(large);
+        check(g.fits(large) && g.set().size() == 19, "layers taken after a failed allocation", k, 0, 0);
+        fit(small);
+        check(g.set().capacity(0) == 4 * 4 * 4 * 32, "a smaller grid gives the memory back", k, 0, 0);
     }
     std::printf("%s: %d failures\n", failures ? "failed" : "ok", failures);
     return failures ? 1 : 0;
