@@ -491,9 +491,13 @@ LHI_API int lhi_net_forward_host(lhi_net* net, const int32_t dims[3], const floa
     if (!net || !r || !type || !z) return fail(LHI_E_INVALID_ARG, "null argument");
     return guarded([&]() -> int {
         const long long n = net_dims_check(dims);
+        const int dd[3] = {dims[0], dims[1], dims[2]};
+        // every allocation before the first copy; whatever fails after it, no copy still reads the caller's
+        // arrays (page-locked ones are read behind the host) when the call returns
+        net->impl->reserve(dd, net->impl->sparse_enabled_);
+        const lhi::OnError settle([net] { cudaStreamSynchronize(net->stream); });
         NetStaging& d = net->staging;
         net_upload(d, n, r, type, solid, nullptr, net->stream);
-        const int dd[3] = {dims[0], dims[1], dims[2]};
         if (net->impl->sparse_enabled_) net->impl->plan_sparse(dd, d.type, net->stream);
         net->impl->forward(dd, d.r, d.type, solid ? d.solid : nullptr, d.z, scale, net->stream, true);
         LHI_CUDA(cudaMemcpyAsync(z, d.z, sizeof(float) * n, cudaMemcpyDeviceToHost, net->stream));
@@ -512,9 +516,11 @@ LHI_API int lhi_net_backward_host(lhi_net* net, const int32_t dims[3], const flo
     if (!net || !r || !type || !dz || !grad) return fail(LHI_E_INVALID_ARG, "null argument");
     return guarded([&]() -> int {
         const long long n = net_dims_check(dims);
+        const int dd[3] = {dims[0], dims[1], dims[2]};
+        net->impl->reserve(dd, false);  // as in the forward call
+        const lhi::OnError settle([net] { cudaStreamSynchronize(net->stream); });
         NetStaging& d = net->staging;
         net_upload(d, n, r, type, solid, dz, net->stream);
-        const int dd[3] = {dims[0], dims[1], dims[2]};
         net->impl->zero_grad(net->stream);
         net->impl->forward(dd, d.r, d.type, solid ? d.solid : nullptr, d.z, scale, net->stream);
         net->impl->backward(d.dz, net->stream);

@@ -1318,6 +1318,13 @@ void LearnedNet::ensure(const int dims[3]) {
     b_ = b;
 }
 
+void LearnedNet::reserve(const int dims[3], bool plan) {
+    ensure(dims);
+    if (!plan) return;
+    if (!plan_mem_.holds(plan_bytes(net_levels(dims)))) plan_type_ = nullptr;  // the lists go
+    plan_mem_.fit(plan_bytes(net_levels(dims)));
+}
+
 void LearnedNet::format_weights(cudaStream_t s) {
     for (int l = 0; l < kNetLayers; ++l) {
         const long long n = (long long)kNetTaps * pad16(kNetCout[l]) * pad16(kNetCin[l]);
@@ -1463,13 +1470,12 @@ void launch_wgrad(const uint16_t* g, int cout, int cout_real, const uint16_t* in
 //   conv0 out H0                     (T0)   a0 needed on dil(H0): computed everywhere
 // Masks: level 0 A, B; level 1 P, Q; level 2 U, W.
 void LearnedNet::plan_sparse(const int dims[3], const uint8_t* type, cudaStream_t s) {
-    ensure(dims);
+    plan_type_ = nullptr;  // no plan until this one is complete
+    reserve(dims, true);
     const int* d0 = b_.dims[0];
     const int* d1 = b_.dims[1];
     const int* d2 = b_.dims[2];
     const long long V0 = b_.vox[0];
-    plan_type_ = nullptr;  // no plan until this one is complete
-    plan_mem_.fit(plan_bytes(net_levels(dims)));
     size_t m = 0;
     for (auto& p : mask_) p = plan_mem_.at<uint8_t>(m++);
     for (auto& p : tflag_) p = plan_mem_.at<uint8_t>(m++);

@@ -157,6 +157,7 @@ public:
     unsigned* counter_ = nullptr;
 
     void ensure(const int dims[3]);
+    void reserve(const int dims[3], bool plan);  // every buffer a forward on this grid uses, its plan's too if asked
     void format_weights(cudaStream_t s);
 
     // sparse evaluation (plan_sparse): voxel masks (level 0: two, level 1:

@@ -5,9 +5,25 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <exception>
 #include <vector>
 
 namespace lhi {
+
+// Runs f when an exception leaves the scope.
+template <class F> class OnError {
+public:
+    explicit OnError(F f) : f_(f), before_(std::uncaught_exceptions()) {}
+    OnError(const OnError&) = delete;
+    OnError& operator=(const OnError&) = delete;
+    ~OnError() {
+        if (std::uncaught_exceptions() > before_) f_();
+    }
+
+private:
+    F f_;
+    int before_;
+};
 
 // Buffers from Mem (void* take(size_t), which throws; void give(void*)), each
 // with a capacity of its own.  fit() keeps the set while every buffer holds

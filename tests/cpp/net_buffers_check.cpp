@@ -4,7 +4,8 @@
 // (counted here from the kernels' own indices, voxel by voxel), also where
 // the grids have equal volume; a set of buffers is whole or empty after a
 // failed allocation, and a network's layers are then no grid's, so that the
-// next call takes them again instead of using what is missing.  Built and run by tests/test_cpu_net_buffers.py.
+// next call takes them again instead of using what is missing; OnError runs
+// on an exception alone.  Built and run by tests/test_cpu_net_buffers.py.
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -123,6 +124,18 @@ int main() {
         fit(small);
         check(g.set().capacity(0) == 4 * 4 * 4 * 32, "a smaller grid gives the memory back", k, 0, 0);
     }
+    int ran = 0;
+    {
+        OnError quiet([&] { ++ran; });
+    }
+    check(ran == 0, "OnError without an error", ran, 0, 0);
+    try {
+        OnError loud([&] { ++ran; });
+        throw std::bad_alloc();
+    } catch (const std::bad_alloc&) {
+        OnError handled([&] { ran += 10; });
+    }
+    check(ran == 1, "OnError with one", ran, 0, 0);
     std::printf("%s: %d failures\n", failures ? "failed" : "ok", failures);
     return failures ? 1 : 0;
 }
