@@ -85,6 +85,7 @@ int fail(int code, const std::string& msg) {
 }
 
 int from_cuda(const lhi::CudaError& e) {
+    cudaGetLastError();  // reported here; the next call's launch checks start from a clear status
     int code = (e.code == cudaErrorMemoryAllocation) ? LHI_E_OOM : LHI_E_CUDA;
     return fail(code, e.what());
 }
