@@ -127,13 +127,19 @@ template <class C, class T, class V> __device__ __forceinline__ C ax7(const Cell
     return r;
 }
 
+// A cell's new z from its old one and the quotient (PressureSolver.cpp:830-834),
+// the roundings written out so that every kernel has the same
+template <class T> __device__ __forceinline__ T smooth_update(T zc, T term, T w, int variant) {
+    if (variant == LHI_SMOOTHER_DAMPED_GS) return fma(w, term, zc);
+    if constexpr (sizeof(T) == 8) return fma(w, term, X<T>::mul(T(1) - w, zc));
+    else return T(fma(1.0 - double(w), double(zc), double(X<T>::mul(w, term))));
+}
+
 // CGSolver<3>::Smooth update of one cell from its loaded row (PressureSolver.cpp:830-834)
 template <class T>
 __device__ __forceinline__ bool smooth7(const Cell7<T, T>& s, T rv, T w, int variant, T& out) {
     if (is_small(s.d)) return false;
-    const T term = (rv - ax7<T>(s)) / s.d;
-    if (variant == LHI_SMOOTHER_DAMPED_GS) out = s.zc + w * term;
-    else out = T((1.0 - double(w)) * double(s.zc) + double(T(w * term)));
+    out = smooth_update(s.zc, (rv - ax7<T>(s)) / s.d, w, variant);
     return true;
 }
 
@@ -958,9 +964,21 @@ template <class T> constexpr int kVecs = int(8 * sizeof(T) / 16);
 template <class T> __host__ __device__ constexpr int row_bytes(int items) { return items * (16 * kVecs<T> + 4); }
 // flags: the diagonal is not small (the sweeps update the cell); the slot
 // holds a cell; its plane is the slab's first / last with a neighbour CTA on
-// that side; the reciprocal of its diagonal is not a normal number.  Bits 16 and up: the cell's index in the slab's z.
-constexpr unsigned kUpdate = 1, kCell = 2, kLeft = 4, kRight = 8, kSlow = 16;
+// that side; the cell has a row (it is not air); neighbours +x, -x, +y, -y,
+// +z, -z of the row; its diagonal lies beyond kMaxDiag.  Bits 16 and up: the
+// cell's index in the slab's z.
+constexpr unsigned kUpdate = 1, kCell = 2, kLeft = 4, kRight = 8, kRow = 16, kNeighbour = 32, kSlow = 32 << 6;
 constexpr int kIndexShift = 16;
+// ClusterSlots::quotient rounds correctly from numerators of kMinNum to kMaxNum
+// under diagonals of at most kMaxDiag (and at least is_small's bound): the
+// remainders are then multiples of the least positive number, the quotient a
+// normal one.  Smaller numerators are scaled by kScale first.
+template <class T> constexpr T kMinNum = sizeof(T) == 4 ? T(0x1p-98) : T(0x1p-900);
+template <class T> constexpr T kMaxNum = sizeof(T) == 4 ? T(0x1p98) : T(0x1p900);
+template <class T> constexpr T kMaxDiag = sizeof(T) == 4 ? T(0x1p26) : T(0x1p100);
+template <class T> constexpr T kScale = sizeof(T) == 4 ? T(0x1p96) : T(0x1p1000);
+// half of the least positive number, scaled
+template <class T> constexpr T kHalfLeast = sizeof(T) == 4 ? T(0x1p-54) : T(0x1p-75);
 }  // namespace cl
 
 template <class T> struct ClusterLevel {
@@ -1025,17 +1043,23 @@ __global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, Cluste
         m = cl::kCell | (unsigned((p + 1) * sx + y * sy + z) << cl::kIndexShift);
         if (L.type[i] != 0) {  // an air cell's row is empty
             const T d = L.diag[i];
+            m |= cl::kRow;
             w[0] = -d;
-            if (x + 1 < L.nx && L.type[i + sx] == 2) w[1] = -L.cx[i];
-            if (x > 0 && L.type[i - sx] == 2) w[2] = -L.cx[i - sx];
-            if (y + 1 < L.ny && L.type[i + sy] == 2) w[3] = -L.cy[i];
-            if (y > 0 && L.type[i - sy] == 2) w[4] = -L.cy[i - sy];
-            if (z + 1 < L.nz && L.type[i + 1] == 2) w[5] = -L.cz[i];
-            if (z > 0 && L.type[i - 1] == 2) w[6] = -L.cz[i - 1];
+            const bool on[6] = {x + 1 < L.nx && L.type[i + sx] == 2, x > 0 && L.type[i - sx] == 2,
+                                y + 1 < L.ny && L.type[i + sy] == 2, y > 0 && L.type[i - sy] == 2,
+                                z + 1 < L.nz && L.type[i + 1] == 2,  z > 0 && L.type[i - 1] == 2};
+            if (on[0]) w[1] = -L.cx[i];
+            if (on[1]) w[2] = -L.cx[i - sx];
+            if (on[2]) w[3] = -L.cy[i];
+            if (on[3]) w[4] = -L.cy[i - sy];
+            if (on[4]) w[5] = -L.cz[i];
+            if (on[5]) w[6] = -L.cz[i - 1];
+#pragma unroll
+            for (int e = 0; e < 6; ++e) m |= on[e] ? cl::kNeighbour << e : 0u;
             if (!is_small(d)) {
                 m |= cl::kUpdate;
                 w[7] = X<T>::div(T(1), d);
-                if (!(fabs(d) < T(1e37))) m |= cl::kSlow;
+                if (!(fabs(d) <= cl::kMaxDiag<T>)) m |= cl::kSlow;
             }
         }
         if (C.ctas > 1 && p == 0 && x > 0) m |= cl::kLeft;
@@ -1050,8 +1074,81 @@ __global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, Cluste
     reinterpret_cast<uint32_t*>(row + size_t(cl::kVecs<T>) * C.items * 16)[q] = m;
 }
 
-// The division of the rare operands (see ClusterSlots::term).
-template <class T> __device__ __noinline__ T cluster_div(T n, T d) { return X<T>::div(n, d); }
+// Copies of a slot's z in the neighbouring CTAs' halo planes: the first
+// plane goes after the left CTA's last (which holds `planes` planes), the
+// last one before the right CTA's first.
+struct ClusterSides {
+    uint32_t left, right;  // z index 0's address in the neighbours, moved by the slab
+};
+template <class T>
+__device__ __forceinline__ ClusterSides cluster_sides(const ClusterLevel<T>& L, unsigned rank, const T* z) {
+    ClusterSides o{0, 0};
+    if (L.ctas > 1) {
+        const int slab = L.planes * L.ny * L.nz * int(sizeof(T));
+        if (rank > 0) o.left = map_rank(smem_addr(z), rank - 1) + slab;
+        if (int(rank) + 1 < L.ctas) o.right = map_rank(smem_addr(z), rank + 1) - slab;
+    }
+    return o;
+}
+template <class T> __device__ __forceinline__ void cluster_push(const ClusterSides& o, unsigned m, int a, T v) {
+    if (m & (cl::kLeft | cl::kRight)) {
+        if (m & cl::kLeft) st_cluster(o.left + a * int(sizeof(T)), v);
+        if (m & cl::kRight) st_cluster(o.right + a * int(sizeof(T)), v);
+    }
+}
+
+template <class T>
+__device__ __forceinline__ const unsigned char* cluster_rows(const ClusterLevel<T>& L, int cta, const T* sm, int c) {
+    const unsigned char* rows = L.rowoff >= 0 ? reinterpret_cast<const unsigned char*>(sm) + L.rowoff
+                                              : L.rows + size_t(cta) * 2 * cl::row_bytes<T>(L.items);
+    return rows + c * cl::row_bytes<T>(L.items);
+}
+
+// The residual of slot q of a colour as the tile kernels form it for every
+// operand: an absent neighbour is not read (0 times an infinity there is not
+// 0).  d: the cell's diagonal.
+template <class T>
+__device__ __forceinline__ T cluster_exact(const ClusterLevel<T>& L, int cta, int c, int q, T rv, T& d) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const T* sm = reinterpret_cast<const T*>(smem);
+    const unsigned char* row = cluster_rows(L, cta, sm, c);
+    const unsigned m = reinterpret_cast<const uint32_t*>(row + size_t(cl::kVecs<T>) * L.items * 16)[q];
+    T w[8];
+#pragma unroll
+    for (int v = 0; v < cl::kVecs<T>; ++v) {
+        const uint4 u = reinterpret_cast<const uint4*>(row)[v * L.items + q];
+        memcpy(&w[v * (16 / int(sizeof(T)))], &u, 16);
+    }
+    const int sy = L.nz, sx = L.ny * L.nz, step[6] = {sx, -sx, sy, -sy, 1, -1};
+    const T* z = sm + L.zoff + (m >> cl::kIndexShift);
+    d = -w[0];
+    T ax = T(0);
+    if (m & cl::kRow) {
+        ax = X<T>::mul(z[0], d);
+#pragma unroll
+        for (int e = 0; e < 6; ++e)
+            if (m & (cl::kNeighbour << e)) ax = fma(z[step[e]], -w[1 + e], ax);
+    }
+    return X<T>::sub(rv, ax);
+}
+// For the operands that ClusterSlots leaves to them: the residual, and a
+// sweep's update of the cell (m: its flags) and of its copies.
+template <class T>
+__device__ __noinline__ T cluster_exact_residual(const ClusterLevel<T>& L, int cta, int c, int q, T rv) {
+    T d;
+    return cluster_exact(L, cta, c, q, rv, d);
+}
+template <class T>
+__device__ __forceinline__ void cluster_exact_update(const ClusterLevel<T>& L, int cta, int c, int q, T rv, unsigned m,
+                                                     T w, int variant) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    T* z = reinterpret_cast<T*>(smem) + L.zoff;
+    const int a = int(m >> cl::kIndexShift);
+    T d;
+    const T res = cluster_exact(L, cta, c, q, rv, d);
+    z[a] = smooth_update(z[a], X<T>::div(res, d), w, variant);
+    cluster_push(cluster_sides(L, unsigned(cta), z), m, a, z[a]);
+}
 
 // Rows of a thread's slots: NK of each colour, in groups of W.
 template <class T, int NK> struct ClusterSlots {
@@ -1060,19 +1157,17 @@ template <class T, int NK> struct ClusterSlots {
     using P = typename V::P;
     P nd[2][G], y[2][G], r[2][G], nc[2][G][6];  // -d, 1 / d, r, -c
     unsigned m[2][NK];
-    bool slow;  // a slot of this thread needs the division
+    bool slow;  // a diagonal of this thread's is beyond kMaxDiag
     __device__ __forceinline__ int a(int c, int k) const { return int(m[c][k] >> cl::kIndexShift); }
 
     __device__ __forceinline__ void load(const ClusterLevel<T>& L, int cta, const T* __restrict__ sm, bool r_global) {
         slow = false;
-        const unsigned char* rows = L.rowoff >= 0 ? reinterpret_cast<const unsigned char*>(sm) + L.rowoff
-                                                  : L.rows + size_t(cta) * 2 * cl::row_bytes<T>(L.items);
         const int sx = L.ny * L.nz;
         const T* rg = L.r + (size_t(cta) * L.planes - 1) * sx;
         const T* rs = sm + L.roff - sx;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            const unsigned char* row = rows + c * cl::row_bytes<T>(L.items);
+            const unsigned char* row = cluster_rows(L, cta, sm, c);
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 T w[W][8], rv[W];
@@ -1109,7 +1204,7 @@ template <class T, int NK> struct ClusterSlots {
     }
 
     // r - A z of group g of a colour, in ax7's order on negated coefficients (the same roundings); an absent
-    // neighbour adds 0 (its coefficient).  zc: the cells' own z.
+    // neighbour adds 0 (its coefficient), or makes the result NaN where its z is not finite.  zc: the cells' own z.
     __device__ __forceinline__ P residual(int c, int g, const T* z, int sx, int sy, P& zc) const {
         T v[7][W];
 #pragma unroll
@@ -1136,47 +1231,62 @@ template <class T, int NK> struct ClusterSlots {
     // Res. Dev. 34(1), 1990: a quotient within one unit in the last place,
     // corrected by its exact remainder times the correctly rounded
     // reciprocal, is the rounded quotient).  Five dependent multiply-adds,
-    // two cells at a time, instead of a division each.  The remainders are
-    // exact down to |n| of about 1e-30 in single precision (below, the
-    // quotient stays within two units in the last place); diagonals whose
-    // reciprocal leaves the normal range take the division.
-    __device__ __forceinline__ P term(int c, int g, P n) const {
-        if (slow) {
-            T nv[W], dv[W], qv[W];
-            V::unpack(n, nv);
-            V::unpack(nd[c][g], dv);
-#pragma unroll
-            for (int j = 0; j < W; ++j) qv[j] = (m[c][g * W + j] & cl::kUpdate) ? cluster_div<T>(nv[j], -dv[j]) : T(0);
-            return V::pack(qv);
-        }
+    // two cells at a time, instead of a division each.  Holds for operands
+    // that rare() does not name.
+    __device__ __forceinline__ P quotient(int c, int g, P n) const {
         const P q0 = V::mul(n, y[c][g]);
         const P q1 = V::fmadd(V::fmadd(nd[c][g], q0, n), y[c][g], q0);
         return V::fmadd(V::fmadd(nd[c][g], q1, n), y[c][g], q1);
     }
-};
 
-// Copies of a slot's z in the neighbouring CTAs' halo planes: the first
-// plane goes after the left CTA's last (which holds `planes` planes), the
-// last one before the right CTA's first.
-struct ClusterSides {
-    uint32_t left, right;  // z index 0's address in the neighbours, moved by the slab
+    // rare: one of the group's numerators lies outside kMinNum .. kMaxNum and
+    // is not 0 (less one, the pattern of 0 is the largest), or a diagonal of
+    // the thread is too large.  Tested on bit patterns, off the quotients'
+    // chain and behind the stores, so that no pass waits for it (comparisons
+    // of every numerator within the chain: 0.06 us of a 0.26 us pass).  Solves
+    // do meet such numerators, where z decays through air gaps, so they have a
+    // path of their own: 93 x 70 x 61 115 us an iteration, 120 to 130 with
+    // all of them through cluster_exact_update, 112 with wrong last bits.
+    static __device__ __forceinline__ unsigned key(float n) { return 2u * __float_as_uint(n); }
+    static __device__ __forceinline__ unsigned key(double n) {
+        return 2u * unsigned(__double2hiint(n)) | unsigned(__double2loint(n) != 0);
+    }
+    static __device__ __forceinline__ bool small(T n) { return key(n) - 1u < key(cl::kMinNum<T>) - 1u; }
+    __device__ __forceinline__ bool rare(P n) const {
+        T nv[W];
+        V::unpack(n, nv);
+        unsigned least = ~0u, most = 0u;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            least = min(least, key(nv[j]) - 1u);
+            most = max(most, key(nv[j]));
+        }
+        return least < key(cl::kMinNum<T>) - 1u || most > key(cl::kMaxNum<T>) || slow;
+    }
+    // The group's quotients q again where numerators are small: scaled by a
+    // power of two they round as the others; scaled back they are exact where
+    // they are normal numbers, and below rounded once more, which differs from
+    // one rounding only where the scaled quotient lies half-way between two
+    // numbers.  exact: the lanes left to cluster_exact_update.
+    __device__ __forceinline__ P scaled_quotient(int c, int g, P n, P q, unsigned& exact) const {
+        const T up[2] = {cl::kScale<T>, cl::kScale<T>}, down[2] = {T(1) / cl::kScale<T>, T(1) / cl::kScale<T>};
+        const P large = quotient(c, g, V::mul(n, V::pack(up))), back = V::mul(large, V::pack(down));
+        T nv[W], qv[W], lv[W], bv[W];
+        V::unpack(n, nv);
+        V::unpack(q, qv);
+        V::unpack(large, lv);
+        V::unpack(back, bv);
+        exact = 0u;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            const bool once = fabs(lv[j] - bv[j] * cl::kScale<T>) != cl::kHalfLeast<T>;
+            const bool ok = !(m[c][g * W + j] & cl::kSlow) && (small(nv[j]) ? once : key(nv[j]) <= key(cl::kMaxNum<T>));
+            if (small(nv[j])) qv[j] = bv[j];
+            if (!ok && (m[c][g * W + j] & cl::kUpdate)) exact |= 1u << j;
+        }
+        return V::pack(qv);
+    }
 };
-template <class T>
-__device__ __forceinline__ ClusterSides cluster_sides(const ClusterLevel<T>& L, unsigned rank, const T* z) {
-    ClusterSides o{0, 0};
-    if (L.ctas > 1) {
-        const int slab = L.planes * L.ny * L.nz * int(sizeof(T));
-        if (rank > 0) o.left = map_rank(smem_addr(z), rank - 1) + slab;
-        if (int(rank) + 1 < L.ctas) o.right = map_rank(smem_addr(z), rank + 1) - slab;
-    }
-    return o;
-}
-template <class T> __device__ __forceinline__ void cluster_push(const ClusterSides& o, unsigned m, int a, T v) {
-    if (m & (cl::kLeft | cl::kRight)) {
-        if (m & cl::kLeft) st_cluster(o.left + a * int(sizeof(T)), v);
-        if (m & cl::kRight) st_cluster(o.right + a * int(sizeof(T)), v);
-    }
-}
 
 // Ends a step of level l: the cluster's barrier, or that of CTA 0's warps
 // that have cells of the level.  Every level has a CTA barrier of its own:
@@ -1185,7 +1295,6 @@ template <class T> __device__ __forceinline__ void cluster_push(const ClusterSid
 static_assert(kMaxLevels + 1 <= 16, "a hardware barrier per level beside __syncthreads's");
 __device__ __forceinline__ void cluster_step(bool wide, int l, int threads) {
     if (wide) cluster_barrier();
-
     else asm volatile("bar.sync %0, %1;" ::"r"(l + 1), "r"(threads) : "memory");
 }
 
@@ -1253,24 +1362,44 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
                     P zc;
-                    const P t = s.term(cc, g, s.residual(cc, g, z, sx, sy, zc));
-                    T out[W];
-                    if (variant == LHI_SMOOTHER_DAMPED_GS) {
-                        V::unpack(V::fmadd(wp, t, zc), out);
-                    } else {
-                        T tv[W], zv[W];
-                        V::unpack(t, tv);
-                        V::unpack(zc, zv);
+                    const P res = s.residual(cc, g, z, sx, sy, zc);
+                    const P t = s.quotient(cc, g, res);
+                    auto store = [&](P q, unsigned skip) {
+                        T out[W];
+                        if (variant == LHI_SMOOTHER_DAMPED_GS) {
+                            V::unpack(V::fmadd(wp, q, zc), out);
+                        } else {
+                            T tv[W], zv[W];
+                            V::unpack(q, tv);
+                            V::unpack(zc, zv);
 #pragma unroll
-                        for (int j = 0; j < W; ++j)
-                            out[j] = T((1.0 - double(w)) * double(zv[j]) + double(X<T>::mul(w, tv[j])));
-                    }
+                            for (int j = 0; j < W; ++j) out[j] = smooth_update(zv[j], tv[j], w, variant);
+                        }
 #pragma unroll
-                    for (int j = 0; j < W; ++j) {
-                        const unsigned m = s.m[cc][g * W + j];
-                        if (m & cl::kUpdate) {
-                            z[s.a(cc, g * W + j)] = out[j];
-                            cluster_push(side, m, s.a(cc, g * W + j), out[j]);
+                        for (int j = 0; j < W; ++j) {
+                            const unsigned m = s.m[cc][g * W + j];
+                            if ((m & cl::kUpdate) && !(skip >> j & 1u)) {
+                                z[s.a(cc, g * W + j)] = out[j];
+                                cluster_push(side, m, s.a(cc, g * W + j), out[j]);
+                            }
+                        }
+                    };
+                    store(t, 0u);
+                    if (s.rare(res)) {  // again, behind the stores; the neighbours' z is the other colour's
+                        unsigned exact;
+                        store(s.scaled_quotient(cc, g, res, t, exact), exact);
+                        if (exact) {
+                            T zv[W], rv[W];
+                            V::unpack(zc, zv);
+                            V::unpack(s.r[cc][g], rv);
+#pragma unroll
+                            for (int j = 0; j < W; ++j)
+                                if (exact >> j & 1u) {
+                                    z[s.a(cc, g * W + j)] = zv[j];
+                                    cluster_exact_update<T>(F, int(rank), cc,
+                                                            int(threadIdx.x) + (g * W + j) * cl::kThreads, rv[j],
+                                                            s.m[cc][g * W + j], w, variant);
+                                }
                         }
                     }
                 }
@@ -1295,8 +1424,15 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
             T rv[W];
             V::unpack(s.residual(cc, g, z, sx, sy, zc), rv);
 #pragma unroll
-            for (int j = 0; j < W; ++j)
-                if (s.m[cc][g * W + j] & cl::kCell) res[s.a(cc, g * W + j)] = rv[j];
+            for (int j = 0; j < W; ++j) {
+                if (!(s.m[cc][g * W + j] & cl::kCell)) continue;
+                if (rv[j] != rv[j]) {
+                    T ro[W];
+                    V::unpack(s.r[cc][g], ro);
+                    rv[j] = cluster_exact_residual<T>(F, int(rank), cc, int(threadIdx.x) + (g * W + j) * cl::kThreads, ro[j]);
+                }
+                res[s.a(cc, g * W + j)] = rv[j];
+            }
         }
     // a coarse plane's children can lie in two slabs where the slabs have an odd number of planes
     if (wide && !(F.planes & 1)) __syncthreads();
