@@ -428,6 +428,7 @@ public:
     int coarse_level_ = 0;   // first level solved by the cluster's coarse kernel (nlev_ if none)
     size_t coarse_smem_ = 0; // its dynamic shared memory
     int coarse_ctas_ = 1;    // CTAs of its cluster
+    bool coarse_swap_ = false;  // its slabs are planes of y, not of x
     void* coarse_rows_ = nullptr;  // the coarse levels' rows in the order its threads read them
     long long coarse_rows_n_ = 0;
     bool spmv_tma_ = false;

@@ -931,7 +931,7 @@ __global__ void __launch_bounds__(kTileThreads) k_prolong_t(int fnx, int fny, in
 
 // ------------------------------------------------- coarse levels in a cluster
 // The V-cycle of the coarse levels [first, last] in one launch, on one
-// cluster of up to 16 CTAs.  A level is cut into slabs of x planes, one per
+// cluster of up to 16 CTAs.  A level is cut into slabs of planes, one per
 // CTA; z, r and the residuals live in the CTAs' shared memory, each slab of z
 // with a copy of the neighbouring CTAs' adjacent planes.  Every thread owns
 // at most kSlots cells of each colour of its slab and keeps their rows
@@ -981,10 +981,12 @@ template <class T> constexpr T kScale = sizeof(T) == 4 ? T(0x1p96) : T(0x1p1000)
 template <class T> constexpr T kHalfLeast = sizeof(T) == 4 ? T(0x1p-54) : T(0x1p-75);
 }  // namespace cl
 
+// A level in its slabs' axes: planes of x over (y, z), or (SWAP) planes of y
+// over (x, z).
 template <class T> struct ClusterLevel {
-    int nx, ny, nz;
+    int nx, ny, nz;  // extent along the planes' axis, along the other one, along z
     int ctas;    // CTAs of the level: 1 (CTA 0 alone) or the whole cluster
-    int planes;  // x planes per CTA
+    int planes;  // planes per CTA
     int hz;      // cells of one colour per row, rounded up
     int items;   // slots of one colour per CTA: planes * ny * hz, rounded up to 4
     int zoff;    // z in shared memory: planes + 2 planes
@@ -993,6 +995,12 @@ template <class T> struct ClusterLevel {
     unsigned char* rows;  // [ctas][2 colours][row_bytes(items)]
     T* r;
     T* z;
+    // index in the level's arrays of cell a (plane 0 lies before the slab) of the slab that starts at plane x0
+    template <bool SWAP> __device__ __forceinline__ long long global(int a, int x0) const {
+        if (!SWAP) return (long long)(x0 - 1) * (ny * nz) + a;
+        const int p = a / (ny * nz), rem = a - p * (ny * nz), y = rem / nz;
+        return ((long long)y * nx + (x0 - 1 + p)) * nz + (rem - y * nz);
+    }
 };
 
 template <class T> struct ClusterLevels {
@@ -1020,7 +1028,7 @@ template <class T> struct ClusterMatrix {
     LevelK<T> L[kMaxLevels];
 };
 template <class T>
-__global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, ClusterMatrix<T> A) {
+__global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, ClusterMatrix<T> A, int swap) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     int l = c.first;
     for (; l <= c.last; ++l) {
@@ -1035,12 +1043,16 @@ __global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, Cluste
     const int cta = half >> 1, colour = half & 1;
     const int sy = L.nz, sx = L.ny * L.nz;
     T w[8] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
-    unsigned m = unsigned(sx) << cl::kIndexShift;  // an empty slot still points into the slab
+    unsigned m = unsigned(C.ny * C.nz) << cl::kIndexShift;  // an empty slot still points into the slab
     int p, y, z;
     if (cluster_slot(C, cta, colour, q, p, y, z)) {
-        const int x = cta * C.planes + p;
+        const int plane = cta * C.planes + p;
+        m = cl::kCell | (unsigned((p + 1) * (C.ny * C.nz) + y * C.nz + z) << cl::kIndexShift);
+        if (C.ctas > 1 && p == 0 && plane > 0) m |= cl::kLeft;
+        if (C.ctas > 1 && p == C.planes - 1 && plane + 1 < C.nx) m |= cl::kRight;
+        const int x = swap ? y : plane;
+        if (swap) y = plane;
         const int i = x * sx + y * sy + z;
-        m = cl::kCell | (unsigned((p + 1) * sx + y * sy + z) << cl::kIndexShift);
         if (L.type[i] != 0) {  // an air cell's row is empty
             const T d = L.diag[i];
             m |= cl::kRow;
@@ -1062,8 +1074,6 @@ __global__ void __launch_bounds__(256) k_cluster_rows(ClusterLevels<T> c, Cluste
                 if (!(fabs(d) <= cl::kMaxDiag<T>)) m |= cl::kSlow;
             }
         }
-        if (C.ctas > 1 && p == 0 && x > 0) m |= cl::kLeft;
-        if (C.ctas > 1 && p == C.planes - 1 && x + 1 < L.nx) m |= cl::kRight;
     }
     unsigned char* row = C.rows + size_t(half) * cl::row_bytes<T>(C.items);
     constexpr int per = 16 / int(sizeof(T));
@@ -1107,7 +1117,7 @@ __device__ __forceinline__ const unsigned char* cluster_rows(const ClusterLevel<
 // The residual of slot q of a colour as the tile kernels form it for every
 // operand: an absent neighbour is not read (0 times an infinity there is not
 // 0).  d: the cell's diagonal.
-template <class T>
+template <class T, bool SWAP>
 __device__ __forceinline__ T cluster_exact(const ClusterLevel<T>& L, int cta, int c, int q, T rv, T& d) {
     extern __shared__ __align__(16) unsigned char smem[];
     const T* sm = reinterpret_cast<const T*>(smem);
@@ -1119,7 +1129,7 @@ __device__ __forceinline__ T cluster_exact(const ClusterLevel<T>& L, int cta, in
         const uint4 u = reinterpret_cast<const uint4*>(row)[v * L.items + q];
         memcpy(&w[v * (16 / int(sizeof(T)))], &u, 16);
     }
-    const int sy = L.nz, sx = L.ny * L.nz, step[6] = {sx, -sx, sy, -sy, 1, -1};
+    const int sx = SWAP ? L.nz : L.ny * L.nz, sy = SWAP ? L.ny * L.nz : L.nz, step[6] = {sx, -sx, sy, -sy, 1, -1};
     const T* z = sm + L.zoff + (m >> cl::kIndexShift);
     d = -w[0];
     T ax = T(0);
@@ -1133,25 +1143,25 @@ __device__ __forceinline__ T cluster_exact(const ClusterLevel<T>& L, int cta, in
 }
 // For the operands that ClusterSlots leaves to them: the residual, and a
 // sweep's update of the cell (m: its flags) and of its copies.
-template <class T>
+template <class T, bool SWAP>
 __device__ __noinline__ T cluster_exact_residual(const ClusterLevel<T>& L, int cta, int c, int q, T rv) {
     T d;
-    return cluster_exact(L, cta, c, q, rv, d);
+    return cluster_exact<T, SWAP>(L, cta, c, q, rv, d);
 }
-template <class T>
+template <class T, bool SWAP>
 __device__ __forceinline__ void cluster_exact_update(const ClusterLevel<T>& L, int cta, int c, int q, T rv, unsigned m,
                                                      T w, int variant) {
     extern __shared__ __align__(16) unsigned char smem[];
     T* z = reinterpret_cast<T*>(smem) + L.zoff;
     const int a = int(m >> cl::kIndexShift);
     T d;
-    const T res = cluster_exact(L, cta, c, q, rv, d);
+    const T res = cluster_exact<T, SWAP>(L, cta, c, q, rv, d);
     z[a] = smooth_update(z[a], X<T>::div(res, d), w, variant);
     cluster_push(cluster_sides(L, unsigned(cta), z), m, a, z[a]);
 }
 
 // Rows of a thread's slots: NK of each colour, in groups of W.
-template <class T, int NK> struct ClusterSlots {
+template <class T, int NK, bool SWAP> struct ClusterSlots {
     static constexpr int W = (sizeof(T) == 4 && NK >= 2) ? 2 : 1, G = NK / W;
     using V = Lanes<T, W>;
     using P = typename V::P;
@@ -1163,7 +1173,6 @@ template <class T, int NK> struct ClusterSlots {
     __device__ __forceinline__ void load(const ClusterLevel<T>& L, int cta, const T* __restrict__ sm, bool r_global) {
         slow = false;
         const int sx = L.ny * L.nz;
-        const T* rg = L.r + (size_t(cta) * L.planes - 1) * sx;
         const T* rs = sm + L.roff - sx;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -1186,7 +1195,7 @@ template <class T, int NK> struct ClusterSlots {
                         memcpy(&w[j][v * (16 / int(sizeof(T)))], &u, 16);
                     }
                     slow |= (m[c][k] & cl::kSlow) != 0;
-                    if (m[c][k] & cl::kCell) rv[j] = r_global ? rg[a(c, k)] : rs[a(c, k)];
+                    if (m[c][k] & cl::kCell) rv[j] = r_global ? L.r[L.template global<SWAP>(a(c, k), cta * L.planes)] : rs[a(c, k)];
                 }
                 T t[W];
                 auto gather = [&](int e) {
@@ -1205,7 +1214,8 @@ template <class T, int NK> struct ClusterSlots {
 
     // r - A z of group g of a colour, in ax7's order on negated coefficients (the same roundings); an absent
     // neighbour adds 0 (its coefficient), or makes the result NaN where its z is not finite.  zc: the cells' own z.
-    __device__ __forceinline__ P residual(int c, int g, const T* z, int sx, int sy, P& zc) const {
+    __device__ __forceinline__ P residual(int c, int g, const T* z, int plane, int row, P& zc) const {
+        const int sx = SWAP ? row : plane, sy = SWAP ? plane : row;  // steps of the grid's x and y
         T v[7][W];
 #pragma unroll
         for (int j = 0; j < W; ++j) {
@@ -1303,12 +1313,12 @@ constexpr int kVisitDown = 0, kVisitLast = 1, kVisitUp = 2;
 // One visit of level l on the way down (smooth, restrict: PressureSolver.cpp:796-819),
 // at the bottom (smooth), or on the way up (prolong: :774-794, smooth).
 // threads: the threads of this CTA that take part (all of them where the level is the cluster's).
-template <class T, int NK>
+template <class T, int NK, bool SWAP>
 __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int mode, unsigned rank, T w, int variant,
                                            int sweeps, int threads) {
     extern __shared__ __align__(16) unsigned char smem[];  // named here too, so that every access is a shared one
     T* sm = reinterpret_cast<T*>(smem);
-    using S = ClusterSlots<T, NK>;
+    using S = ClusterSlots<T, NK, SWAP>;
     using V = typename S::V;
     using P = typename S::P;
     constexpr int W = S::W, G = S::G;
@@ -1396,7 +1406,7 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
                             for (int j = 0; j < W; ++j)
                                 if (exact >> j & 1u) {
                                     z[s.a(cc, g * W + j)] = zv[j];
-                                    cluster_exact_update<T>(F, int(rank), cc,
+                                    cluster_exact_update<T, SWAP>(F, int(rank), cc,
                                                             int(threadIdx.x) + (g * W + j) * cl::kThreads, rv[j],
                                                             s.m[cc][g * W + j], w, variant);
                                 }
@@ -1407,12 +1417,11 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
             cluster_step(wide, l, threads);
         }
     if (mode != kVisitDown) {
-        T* zg = F.z + (long long)(x0 - 1) * sx;
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc)
 #pragma unroll
             for (int k = 0; k < NK; ++k)
-                if (s.m[cc][k] & cl::kCell) zg[s.a(cc, k)] = z[s.a(cc, k)];
+                if (s.m[cc][k] & cl::kCell) F.z[F.template global<SWAP>(s.a(cc, k), x0)] = z[s.a(cc, k)];
         return;
     }
     T* res = sm + c.resoff - sx;
@@ -1429,7 +1438,7 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
                 if (rv[j] != rv[j]) {
                     T ro[W];
                     V::unpack(s.r[cc][g], ro);
-                    rv[j] = cluster_exact_residual<T>(F, int(rank), cc, int(threadIdx.x) + (g * W + j) * cl::kThreads, ro[j]);
+                    rv[j] = cluster_exact_residual<T, SWAP>(F, int(rank), cc, int(threadIdx.x) + (g * W + j) * cl::kThreads, ro[j]);
                 }
                 res[s.a(cc, g * W + j)] = rv[j];
             }
@@ -1446,8 +1455,9 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
         const int Y = rem / C.nz, Z = rem - Y * C.nz;
         T rv[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int p = 2 * X + (k >> 2) - x0, fy = 2 * Y + ((k >> 1) & 1), fz = 2 * Z + (k & 1);
+        for (int k = 0; k < 8; ++k) {  // in the reference's order, x first
+            const int kp = SWAP ? (k >> 1) & 1 : k >> 2, ky = SWAP ? k >> 2 : (k >> 1) & 1;
+            const int p = 2 * X + kp - x0, fy = 2 * Y + ky, fz = 2 * Z + (k & 1);
             const bool next = p >= F.planes;
             const T* src = sm + c.resoff + ((next ? 0 : p) * F.ny + fy) * F.nz + fz;
             if (next) rv[k] = ld_cluster<T>(map_rank(smem_addr(src), rank + 1));
@@ -1455,17 +1465,17 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
         }
         T acc = T(0);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc = T(double(acc) + 0.125 * double(rv[k]));  // the reference's order
+        for (int k = 0; k < 8; ++k) acc = T(double(acc) + 0.125 * double(rv[k]));
         const int own = C.ctas > 1 ? X / C.planes : 0;
         T* dst = sm + C.roff + (X - own * C.planes) * csx + rem;
         if (own == int(rank)) *dst = acc;
         else st_cluster(map_rank(smem_addr(dst), own), acc);
-        C.r[X * csx + rem] = acc;
+        C.r[C.template global<SWAP>(csx + rem, X)] = acc;
     }
     cluster_step(wide, l, threads);  // the next level's r is ready, and no CTA still reads these residuals
 }
 
-template <class T>
+template <class T, bool SWAP>
 __global__ void __launch_bounds__(cl::kThreads, 1)
     k_coarse_cycle(const __grid_constant__ ClusterLevels<T> c, T w, int variant, int pre, int post, int fin,
                    const int* __restrict__ stop) {
@@ -1495,9 +1505,9 @@ __global__ void __launch_bounds__(cl::kThreads, 1)
         const ClusterLevel<T>& L = c.L[l];
         const int threads = L.ctas > 1 ? cl::kThreads : max(32, min(cl::kThreads, (L.items + 31) & ~31));
         if ((L.ctas == 1 && rank != 0) || int(threadIdx.x) >= threads) continue;
-        if (L.items <= cl::kThreads) cluster_visit<T, 1>(c, l, mode, rank, w, variant, sweeps, threads);
-        else if (L.items <= 2 * cl::kThreads) cluster_visit<T, 2>(c, l, mode, rank, w, variant, sweeps, threads);
-        else cluster_visit<T, cl::kSlots<T>>(c, l, mode, rank, w, variant, sweeps, threads);
+        if (L.items <= cl::kThreads) cluster_visit<T, 1, SWAP>(c, l, mode, rank, w, variant, sweeps, threads);
+        else if (L.items <= 2 * cl::kThreads) cluster_visit<T, 2, SWAP>(c, l, mode, rank, w, variant, sweeps, threads);
+        else cluster_visit<T, cl::kSlots<T>, SWAP>(c, l, mode, rank, w, variant, sweeps, threads);
     }
     if (wide) cluster_barrier();  // no CTA leaves while another may still reach its shared memory
 }
@@ -2263,6 +2273,7 @@ template <class T, class TX> void LiquidImpl<T, TX>::build_lhs(double rho, doubl
 // residuals, then the rows of the levels below the first, and the first
 // level's where they still fit (they are read twice a cycle).
 template <class T, class TX> static ClusterLevels<T> coarse_view(const LiquidImpl<T, TX>& s, int first) {
+    const bool swap = s.coarse_swap_;  // slabs of y
     ClusterLevels<T> c{};
     c.first = first;
     c.last = s.nlev_ - 1;
@@ -2271,22 +2282,22 @@ template <class T, class TX> static ClusterLevels<T> coarse_view(const LiquidImp
     for (int l = c.first; l <= c.last; ++l) {
         const LevelDev<T>& D = s.lv_[l];
         ClusterLevel<T>& L = c.L[l];
-        L.nx = D.nx;
-        L.ny = D.ny;
+        L.nx = swap ? D.ny : D.nx;
+        L.ny = swap ? D.nx : D.ny;
         L.nz = D.nz;
         L.hz = (D.nz + 1) / 2;
         // CTA 0 alone where its threads hold the whole level
         const bool solo = (long long)D.nx * D.ny * L.hz <= cl::kThreads;
         L.ctas = solo ? 1 : s.coarse_ctas_;
-        L.planes = (D.nx + L.ctas - 1) / L.ctas;
-        L.items = int(std::min(((long long)L.planes * D.ny * L.hz + 3) / 4 * 4, 1LL << 24));
+        L.planes = (L.nx + L.ctas - 1) / L.ctas;
+        L.items = int(std::min(((long long)L.planes * L.ny * L.hz + 3) / 4 * 4, 1LL << 24));
         L.zoff = int(off);
-        off += (long long)(L.planes + 2) * D.ny * D.nz;
+        off += (long long)(L.planes + 2) * L.ny * L.nz;
         L.rows = rows;
         if (rows) rows += size_t(L.ctas) * 2 * cl::row_bytes<T>(L.items);
         L.r = D.r;
         L.z = D.z;
-        slab = std::max(slab, (long long)L.planes * D.ny * D.nz);
+        slab = std::max(slab, (long long)L.planes * L.ny * L.nz);
     }
     off += 4;
     c.zend = int(off);
@@ -2324,7 +2335,8 @@ template <class T, class TX> void LiquidImpl<T, TX>::build_masks() {
     if (coarse_level_ < nlev_) {
         ClusterMatrix<T> m{};
         for (int l = coarse_level_; l < nlev_; ++l) m.L[l] = lk(lv_[l]);
-        k_cluster_rows<T><<<blocks_for(coarse_rows_n_, 256), 256, 0, cur_>>>(coarse_view(*this, coarse_level_), m);
+        k_cluster_rows<T><<<blocks_for(coarse_rows_n_, 256), 256, 0, cur_>>>(coarse_view(*this, coarse_level_), m,
+                                                                              int(coarse_swap_));
         LHI_LAUNCH_CHECK();
     }
 }
@@ -2471,8 +2483,10 @@ template <class T, class TX> void LiquidImpl<T, TX>::prolong_to(int level) {
 // CTAs of the coarse kernel's cluster (its non-portable maximum where the
 // device has room for one).
 template <class T> static int coarse_cluster_ctas() {
-    LHI_CUDA(cudaFuncSetAttribute(k_coarse_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cl::kSmemBytes)));
-    LHI_CUDA(cudaFuncSetAttribute(k_coarse_cycle<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (const auto k : {k_coarse_cycle<T, false>, k_coarse_cycle<T, true>}) {
+        LHI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cl::kSmemBytes)));
+        LHI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
     for (int n = cl::kMaxCtas; n > 8; n /= 2) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(unsigned(n));
@@ -2485,7 +2499,7 @@ template <class T> static int coarse_cluster_ctas() {
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, k_coarse_cycle<T>, &cfg) == cudaSuccess && fit > 0) return n;
+        if (cudaOccupancyMaxActiveClusters(&fit, k_coarse_cycle<T, false>, &cfg) == cudaSuccess && fit > 0) return n;
         cudaGetLastError();
     }
     return 8;
@@ -2493,20 +2507,33 @@ template <class T> static int coarse_cluster_ctas() {
 
 // Picks the first level (below the finest) from which on every level's slabs
 // fit the cluster: at most coarse_cells cells where the caller set that, and
-// slabs of at most two colours of kSlots cells a thread.
+// slabs of at most two colours of kSlots cells a thread.  Slabs are planes of
+// x, or planes of y where those let a finer level in: a level flat in x is a
+// slab of its own otherwise (1 x 50 x 50 in FP64, 20 sweeps at the bottom of a
+// two-level cycle: 139 us
+// an iteration on the tile kernels, 76 with slabs of y).  The kernel is
+// compiled for either, so that the common one's steps stay in few registers.
 template <class T, class TX> void LiquidImpl<T, TX>::setup_coarse() {
     coarse_level_ = nlev_;
     coarse_smem_ = 0;
     if (nlev_ < 2) return;
     const int ctas = coarse_cluster_ctas<T>();
     const long long slots = (long long)cl::kSlots<T> * cl::kThreads;
-    for (int first = nlev_ - 1; first >= 1; --first) {  // the finest first level that still fits
-        if (sp_.coarse_cells > 0 && lv_[first].n > sp_.coarse_cells) break;
-        coarse_ctas_ = ctas;
-        const ClusterLevels<T> c = coarse_view(*this, first);
-        if (c.L[first].items > slots || coarse_smem(c) > cl::kSmemBytes) break;
-        coarse_level_ = first;
-    }
+    auto finest = [&](bool swap) {  // the finest first level that still fits
+        coarse_swap_ = swap;
+        int fit = nlev_;
+        for (int first = nlev_ - 1; first >= 1; --first) {
+            if (sp_.coarse_cells > 0 && lv_[first].n > sp_.coarse_cells) break;
+            coarse_ctas_ = ctas;
+            const ClusterLevels<T> c = coarse_view(*this, first);
+            if (c.L[first].items > slots || coarse_smem(c) > cl::kSmemBytes) break;
+            fit = first;
+        }
+        return fit;
+    };
+    const int by_y = finest(true), by_x = finest(false);
+    coarse_swap_ = by_y < by_x;
+    coarse_level_ = std::min(by_x, by_y);
     if (coarse_level_ == nlev_) return;
     ClusterLevels<T> c = coarse_view(*this, coarse_level_);
     coarse_ctas_ = c.L[coarse_level_].ctas;
@@ -2559,9 +2586,10 @@ template <class T, class TX> void LiquidImpl<T, TX>::enqueue_vcycle_levels() {
             at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            LHI_CUDA(cudaLaunchKernelEx(&cfg, k_coarse_cycle<T>, coarse_view(*this, coarse_level_), T(sp_.smoothing_factor),
-                                        int(sp_.smoother), int(sp_.num_pre_smooth), int(sp_.num_post_smooth),
-                                        int(sp_.num_final_smooth), static_cast<const int*>(&sc_->stop)));
+            LHI_CUDA(cudaLaunchKernelEx(&cfg, coarse_swap_ ? k_coarse_cycle<T, true> : k_coarse_cycle<T, false>,
+                                        coarse_view(*this, coarse_level_), T(sp_.smoothing_factor), int(sp_.smoother),
+                                        int(sp_.num_pre_smooth), int(sp_.num_post_smooth), int(sp_.num_final_smooth),
+                                        static_cast<const int*>(&sc_->stop)));
             LHI_LAUNCH_CHECK();
         }
         for (int l = Lc - 1; l >= 0; --l) {
