@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kBrThreads) k_conv_brick(const __grid_constant
 // ------------------------------------------------------- weight gradient
 constexpr int kWgChunk = 64;        // voxels per MMA batch (K)
 constexpr int kWgChunksPerCta = 32;  // at most
-constexpr int kWgThreads = 128;
+constexpr int kWgThreads = 128;     // one per row of D
 constexpr int kWgCtas = 4;  // an SM
 
 struct WgradParams {
@@ -672,20 +672,19 @@ template <int COUT, int CIN> __global__ void __launch_bounds__(kWgThreads, kWgCt
     tc_fence_after();
     ok = __all_sync(0xffffffffu, ok);
     if (ok && issued > 0) {
-        // warps w and w + 4 read the rows of quarter w (TMEM lane = row of D), half of the columns each
-        const int row = tid % 128;
-        const uint32_t trow = tmem + (uint32_t(row & ~31) << 16);
-        const int tap = tap0 + row / COUT, co = row % COUT;
-        constexpr int kCols = CIN / (kWgThreads / 128);
-        for (int c0 = (tid / 128) * kCols; c0 < (tid / 128 + 1) * kCols; c0 += 8) {
+        // warp w reads the rows of quarter w (TMEM lane = row of D = thread), all columns
+        const uint32_t trow = tmem + (uint32_t(warp * 32) << 16);
+        const int tap = tap0 + tid / COUT, co = tid % COUT;
+        for (int c0 = 0; c0 < CIN; c0 += 8) {
             float a[8];
             tmem_ld8(trow + c0, a);
-            if (co < P.cout_real && tap < kNetTaps)
+            if (co < P.cout_real && tap < kNetTaps) {
+                float* g = P.grad_w + ((long long)tap * P.cout_real + co) * P.cin_real + c0;
 #pragma unroll
                 for (int k = 0; k < 8; k += 4)  // cin_real and the layer's offset are multiples of 4
                     if (c0 + k < P.cin_real)
-                        atomicAdd(reinterpret_cast<float4*>(P.grad_w + ((long long)tap * P.cout_real + co) * P.cin_real + c0 + k),
-                                  make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]));
+                        atomicAdd(reinterpret_cast<float4*>(g + k), make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]));
+            }
         }
     }
     if (!ok && tid == 0 && atomicExch(&P.status->timeout, 1) == 0) {
@@ -1658,14 +1657,14 @@ void LearnedNet::backward(const float* dz, cudaStream_t s) {
     launch_wgrad(b_.g[2], 64, 64, b_.p1, 32, 32, d2, GW(2), status_, s);
     launch_conv(b_.g[2], 64, WB(2), 32, nullptr, 32, d2, 1, nullptr, 0, nullptr, b_.dx, status_, s);
     // layer 1: dh1 = g3 (skip) + unpool(dp1) / 8
-    k_relu_grad_unpool<<<nb(V1 * 32 / 8), 256, 0, s>>>(b_.g[3], b_.dx, d2[0], d2[1], d2[2], b_.h1, d1[0], d1[1], d1[2], 32,
-                                                    relu_ ? 1 : 0, b_.g[1]);
+    k_relu_grad_unpool<<<nb(V1 * 32 / 8), 256, 0, s>>>(b_.g[3], b_.dx, d2[0], d2[1], d2[2], b_.h1, d1[0], d1[1], d1[2],
+                                                       32, relu_ ? 1 : 0, b_.g[1]);
     LHI_LAUNCH_CHECK();
     launch_wgrad(b_.g[1], 32, 32, b_.p0, 16, 16, d1, GW(1), status_, s);
     launch_conv(b_.g[1], 32, WB(1), 16, nullptr, 16, d1, 1, nullptr, 0, nullptr, b_.dx, status_, s);
     // layer 0: dh0 = g4 (skip) + unpool(dp0) / 8
-    k_relu_grad_unpool<<<nb(V0 * 16 / 8), 256, 0, s>>>(b_.g[4], b_.dx, d1[0], d1[1], d1[2], b_.h0, d0[0], d0[1], d0[2], 16,
-                                                    relu_ ? 1 : 0, b_.g[0]);
+    k_relu_grad_unpool<<<nb(V0 * 16 / 8), 256, 0, s>>>(b_.g[4], b_.dx, d1[0], d1[1], d1[2], b_.h0, d0[0], d0[1], d0[2],
+                                                       16, relu_ ? 1 : 0, b_.g[0]);
     LHI_LAUNCH_CHECK();
     launch_wgrad(b_.g[0], 16, 16, b_.a0, 16, 4, d0, GW(0), status_, s);
 }
