@@ -529,18 +529,7 @@ __global__ void __launch_bounds__(1024) k_tiles_finalize(TileLevels tl, int* __r
 
 // ----------------------------------------------------------- V-cycle
 // CGSolver<3>::Smooth (PressureSolver.cpp:821-837): one colour of damped
-// red-black Gauss-Seidel; (1. - w) * z + w * term evaluated in double.
-template <class T>
-__device__ __forceinline__ void smooth_cell(const LevelK<T>& L, const T* __restrict__ r, T* __restrict__ z, T w,
-                                            int variant, long long i, int x, int y, int zz) {
-    T dg = L.diag[i];
-    if (is_small(dg)) return;
-    T term = (r[i] - ax_at<T>(L, z, i, x, y, zz)) / dg;
-    if (variant == LHI_SMOOTHER_DAMPED_GS) z[i] = z[i] + w * term;
-    else z[i] = T((1.0 - double(w)) * double(z[i]) + double(T(w * term)));
-}
-
-// One colour of one level over its active tiles.  A work unit is one of the
+// red-black Gauss-Seidel on one level's active tiles.  A work unit is one of the
 // four rows y of that colour in a tile, a thread its cell at (x, z).  Latency
 // bounds it: one row a thread takes 40 registers, so that six CTAs an SM are
 // at work (FP64: three); four rows, loaded ahead, took 128 and two CTAs
@@ -678,7 +667,9 @@ __global__ void __launch_bounds__(rb::kThreads, 1)
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
     double v[2] = {0.0, 0.0};  // r.z and Ap.z of the swept tiles (final_dot)
     // the loads that lead to the first copy, all at once (the list has at
-    // least gridDim.x entries whatever the count), and the maps' descriptors
+    // least gridDim.x entries whatever the count), and the maps' descriptors,
+    // before the CTA's barrier: a PCG iteration of 64^3 takes 150 us, 152 with
+    // one after another; 128^3 174 and 176, 192^3 310 and 318, 256^3 the same
     const int stop = sc->stop, units = *count, id0 = ids[blockIdx.x];
     if (threadIdx.x == 0) {
         prefetch_map(&mz);
@@ -1438,7 +1429,8 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
                 if (rv[j] != rv[j]) {
                     T ro[W];
                     V::unpack(s.r[cc][g], ro);
-                    rv[j] = cluster_exact_residual<T, SWAP>(F, int(rank), cc, int(threadIdx.x) + (g * W + j) * cl::kThreads, ro[j]);
+                    rv[j] = cluster_exact_residual<T, SWAP>(F, int(rank), cc,
+                                                            int(threadIdx.x) + (g * W + j) * cl::kThreads, ro[j]);
                 }
                 res[s.a(cc, g * W + j)] = rv[j];
             }
@@ -2435,7 +2427,7 @@ template <class T, class TX> bool LiquidImpl<T, TX>::smooth(int level, int sweep
         }
         return final_dot;
     }
-    const TileK tk = tile_k(L, &sc_->tile_count[level], tile_grid_);
+    const TileK tk{L.tiles, &sc_->tile_count[level], L.tdim[1], L.tdim[2], 1};  // k_sweep splits tiles by itself
     for (int s = 0; s < sweeps; ++s)
         for (int phase = 0; phase < 2; ++phase) {
             auto ps_ = scope(cat);
