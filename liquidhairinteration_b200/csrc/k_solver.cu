@@ -930,11 +930,13 @@ __global__ void __launch_bounds__(kTileThreads) k_prolong_t(int fnx, int fny, in
 // sweeps, so a colour pass loads the neighbours' z from its own shared
 // memory, updates, stores, and pushes the cells of a slab's outer planes
 // into the neighbours' copies through distributed shared memory; a cluster
-// barrier ends the pass.  Levels of one slot a thread run on CTA 0
-// alone, by as many warps as have cells, between CTA barriers: one slot a
-// thread, a pass of 0.3 us against 0.6 us over the cluster (whose barrier
-// with remote stores in flight takes 0.45 us); at 16^3 one CTA's shared
-// memory and issue slots lose (1.0 us a pass against 0.6).
+// barrier ends the pass.  Levels of one group of slots a thread run on CTA 0
+// alone, by as many warps as have cells, between CTA barriers: with one slot
+// a pass of 0.3 us against 0.6 us over the cluster (whose barrier with remote
+// stores in flight takes 0.45 us); at 16^3 one CTA's shared memory and issue
+// slots lose (1.0 us a pass against 0.6).  A warp skips the groups in which it
+// has no cell to update (air above the water: 64^3 5+5 147 us an iteration
+// against 149, 93 x 70 x 61 113 against 115).
 // What bounds it: the instructions and latency of a pass (shared-memory
 // loads, the update's dependent arithmetic, the barrier), not bytes.  In
 // single precision a thread's slots go in pairs through the packed two-wide
@@ -1246,8 +1248,8 @@ template <class T, int NK, bool SWAP> struct ClusterSlots {
     // chain and behind the stores, so that no pass waits for it (comparisons
     // of every numerator within the chain: 0.06 us of a 0.26 us pass).  Solves
     // do meet such numerators, where z decays through air gaps, so they have a
-    // path of their own: 93 x 70 x 61 115 us an iteration, 120 to 130 with
-    // all of them through cluster_exact_update, 112 with wrong last bits.
+    // path of their own (93 x 70 x 61: all of them through
+    // cluster_exact_update cost 8% of an iteration).
     static __device__ __forceinline__ unsigned key(float n) { return 2u * __float_as_uint(n); }
     static __device__ __forceinline__ unsigned key(double n) {
         return 2u * unsigned(__double2hiint(n)) | unsigned(__double2loint(n) != 0);
@@ -1355,53 +1357,55 @@ __device__ __noinline__ void cluster_visit(const ClusterLevels<T>& c, int l, int
 #pragma unroll
     for (int j = 0; j < W; ++j) wv[j] = w;
     const P wp = V::pack(wv);
-    const bool busy = int(threadIdx.x & ~31u) < F.items;  // this warp has slots
+    unsigned wet = 0;  // groups (colour 0's, colour 1's) in which this warp has a cell to update
+#pragma unroll
+    for (int k = 0; k < 2 * NK; ++k)
+        wet |= __any_sync(0xffffffffu, s.m[k / NK][k % NK] & cl::kUpdate) ? 1u << (k / W) : 0u;
     for (int n = 0; n < sweeps; ++n)
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
-            if (busy) {
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    P zc;
-                    const P res = s.residual(cc, g, z, sx, sy, zc);
-                    const P t = s.quotient(cc, g, res);
-                    auto store = [&](P q, unsigned skip) {
-                        T out[W];
-                        if (variant == LHI_SMOOTHER_DAMPED_GS) {
-                            V::unpack(V::fmadd(wp, q, zc), out);
-                        } else {
-                            T tv[W], zv[W];
-                            V::unpack(q, tv);
-                            V::unpack(zc, zv);
+            for (int g = 0; g < G; ++g) {
+                if (!(wet >> (cc * G + g) & 1u)) continue;
+                P zc;
+                const P res = s.residual(cc, g, z, sx, sy, zc);
+                const P t = s.quotient(cc, g, res);
+                auto store = [&](P q, unsigned skip) {
+                    T out[W];
+                    if (variant == LHI_SMOOTHER_DAMPED_GS) {
+                        V::unpack(V::fmadd(wp, q, zc), out);
+                    } else {
+                        T tv[W], zv[W];
+                        V::unpack(q, tv);
+                        V::unpack(zc, zv);
 #pragma unroll
-                            for (int j = 0; j < W; ++j) out[j] = smooth_update(zv[j], tv[j], w, variant);
+                        for (int j = 0; j < W; ++j) out[j] = smooth_update(zv[j], tv[j], w, variant);
+                    }
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        const unsigned m = s.m[cc][g * W + j];
+                        if ((m & cl::kUpdate) && !(skip >> j & 1u)) {
+                            z[s.a(cc, g * W + j)] = out[j];
+                            cluster_push(side, m, s.a(cc, g * W + j), out[j]);
                         }
+                    }
+                };
+                store(t, 0u);
+                if (s.rare(res)) {  // again, behind the stores; the neighbours' z is the other colour's
+                    unsigned exact;
+                    store(s.scaled_quotient(cc, g, res, t, exact), exact);
+                    if (exact) {
+                        T zv[W], rv[W];
+                        V::unpack(zc, zv);
+                        V::unpack(s.r[cc][g], rv);
 #pragma unroll
-                        for (int j = 0; j < W; ++j) {
-                            const unsigned m = s.m[cc][g * W + j];
-                            if ((m & cl::kUpdate) && !(skip >> j & 1u)) {
-                                z[s.a(cc, g * W + j)] = out[j];
-                                cluster_push(side, m, s.a(cc, g * W + j), out[j]);
+                        for (int j = 0; j < W; ++j)
+                            if (exact >> j & 1u) {
+                                z[s.a(cc, g * W + j)] = zv[j];
+                                cluster_exact_update<T, SWAP>(F, int(rank), cc,
+                                                              int(threadIdx.x) + (g * W + j) * cl::kThreads, rv[j],
+                                                              s.m[cc][g * W + j], w, variant);
                             }
-                        }
-                    };
-                    store(t, 0u);
-                    if (s.rare(res)) {  // again, behind the stores; the neighbours' z is the other colour's
-                        unsigned exact;
-                        store(s.scaled_quotient(cc, g, res, t, exact), exact);
-                        if (exact) {
-                            T zv[W], rv[W];
-                            V::unpack(zc, zv);
-                            V::unpack(s.r[cc][g], rv);
-#pragma unroll
-                            for (int j = 0; j < W; ++j)
-                                if (exact >> j & 1u) {
-                                    z[s.a(cc, g * W + j)] = zv[j];
-                                    cluster_exact_update<T, SWAP>(F, int(rank), cc,
-                                                            int(threadIdx.x) + (g * W + j) * cl::kThreads, rv[j],
-                                                            s.m[cc][g * W + j], w, variant);
-                                }
-                        }
                     }
                 }
             }
@@ -2278,8 +2282,11 @@ template <class T, class TX> static ClusterLevels<T> coarse_view(const LiquidImp
         L.ny = swap ? D.nx : D.ny;
         L.nz = D.nz;
         L.hz = (D.nz + 1) / 2;
-        // CTA 0 alone where its threads hold the whole level
-        const bool solo = (long long)D.nx * D.ny * L.hz <= cl::kThreads;
+        // CTA 0 alone where its threads hold the whole level in one group of slots each (FP32: a pair).  8 x 12 x 16
+        // cells at the bottom of a two-level cycle: 68 us an iteration against 72 over the cluster, 12^3 below 24^3:
+        // 91 and 95; in more slots the cluster is better (11 x 14 x 16: 73 and 84, 14^3: 77 and 90, 12^3 in FP64: 106
+        // and 113)
+        const bool solo = (long long)D.nx * D.ny * L.hz <= (sizeof(T) == 4 ? 2 : 1) * cl::kThreads;
         L.ctas = solo ? 1 : s.coarse_ctas_;
         L.planes = (L.nx + L.ctas - 1) / L.ctas;
         L.items = int(std::min(((long long)L.planes * L.ny * L.hz + 3) / 4 * 4, 1LL << 24));

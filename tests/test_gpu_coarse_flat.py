@@ -1,5 +1,6 @@
-"""Coarse levels that are flat in x: the cluster cuts them into slabs of y
-planes where slabs of x planes would not fit.  V-cycles equal the tile
+"""Coarse levels at the edges of how the cluster is shared out: levels flat in
+x, which it cuts into slabs of y planes where slabs of x planes would not fit,
+and levels around the size that its first CTA takes alone.  V-cycles equal the tile
 kernels' bit for bit, as in test_gpu_coarse_cluster.py."""
 import numpy as np
 import pytest
@@ -15,6 +16,9 @@ GRIDS = [((2, 100, 100), 2, "fp64", True), ((2, 100, 100), 3, "fp32", True), ((3
          ((2, 126, 130), 2, "fp32", True), ((2, 128, 128), 3, "fp64", True), ((2, 130, 128), 2, "fp32", True),
          ((4, 200, 64), 3, "fp64", True), ((10, 197, 75), 5, "fp64", True), ((9, 146, 150), 4, "fp32", True),
          ((4, 400, 400), 2, "fp64", False)]
+# level 1 on CTA 0 alone in one and in two slots a thread, at the most cells it takes, and one plane above
+GRIDS += [(g, 3, p, True) for g in ((24, 24, 24), (32, 16, 16), (32, 16, 32), (34, 16, 32), (34, 16, 16))
+          for p in ("fp32", "fp64")]
 
 
 @pytest.mark.parametrize("grid,levels,prec,coarse", GRIDS)
